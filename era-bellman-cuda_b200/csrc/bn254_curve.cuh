@@ -203,7 +203,7 @@ struct curve {
   // XYZZ -> affine for a finite p: one inversion of ZZ ZZZ gives both
   // 1/ZZ = ZZZ / (ZZ ZZZ) and 1/ZZZ = ZZ / (ZZ ZZZ).  Output fully reduced.
   static BN_HD_COLD affine to_affine(const xyzz &p) {
-    const fe inv = fq::inverse(fq::mul(p.zz, p.zzz));
+    const fe inv = fq::to_mont(fq::inverse_binary(fq::from_mont(fq::mul(p.zz, p.zzz))));
     affine a;
     a.x = fq::reduce_full(fq::mul(p.x, fq::mul(p.zzz, inv)));
     a.y = fq::reduce_full(fq::mul(p.y, fq::mul(p.zz, inv)));

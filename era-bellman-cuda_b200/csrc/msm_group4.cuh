@@ -128,4 +128,47 @@ __device__ __forceinline__ xyzz add_group4(const xyzz &p, const xyzz &q) {
   return r;
 }
 
+// fq::inverse_binary shared by a group of four lanes (a standard-form
+// canonical value, the same in all four): the 30 division steps run in every
+// lane, and of the four rows that the matrix is applied to (d and e modulo p,
+// f and g) each lane computes one and swaps it with its neighbour's.  Lanes 0
+// and 1 of a group hold d and e in (x, y), lanes 2 and 3 hold f and g.
+__device__ __forceinline__ fe inverse_group4(const fe &a) {
+  constexpr int WORDS = fq::INV_WORDS;
+  const unsigned lane = threadIdx.x & 31, low = lane & ~3u;
+  const bool second = lane & 1, fg = lane & 2;
+  int32_t x[WORDS], y[WORDS];
+  fq::split30(a, y);
+#pragma unroll
+  for (int i = 0; i < WORDS; i++) {
+    x[i] = fg ? fq::mod30(i) : 0;
+    y[i] = fg ? y[i] : (i == 0);
+  }
+  int32_t theta = 0;
+  for (int round = 0; round < 20; round++) {
+    const uint32_t f0 = (uint32_t)x[0] | (uint32_t)x[1] << 30, g0 = (uint32_t)y[0] | (uint32_t)y[1] << 30;
+    const fq::steps30 m = fq::division_steps(theta, __shfl_sync(0xffffffffu, f0, low + 2), __shfl_sync(0xffffffffu, g0, low + 2));
+    const int32_t u = second ? m.q : m.u, v = second ? m.r : m.v;
+    const int32_t k = fq::multiple30(x, y, u, v);
+    int32_t row[WORDS];
+    fq::combine30(x, y, u, v, fg ? 0 : k, row);
+    int32_t rest = 0;
+#pragma unroll
+    for (int i = 0; i < WORDS; i++) {
+      const int32_t other = __shfl_xor_sync(0xffffffffu, row[i], 1);
+      x[i] = second ? other : row[i];
+      y[i] = second ? row[i] : other;
+      rest |= y[i];
+    }
+    if (__all_sync(0xffffffffu, !fg || rest == 0))
+      break;
+  }
+  const int32_t top = __shfl_sync(0xffffffffu, x[WORDS - 1], low + 2);
+#pragma unroll
+  for (int i = 0; i < WORDS; i++)
+    x[i] = __shfl_sync(0xffffffffu, x[i], low);
+  const fe inverse = fq::join30(x, top < 0 ? -1 : 1);
+  return select_fe(fq::is_zero_exact(a), fq::zero(), inverse);
+}
+
 } // namespace msm_b200

@@ -194,3 +194,17 @@ def test_batched_results(gpu, oracle):
     bc.base_table_destroy(table)
     for p in sd + rd + [kd, bd]:
         bc.free(p)
+
+
+@pytest.mark.parametrize("bits", [[7], [8], [15, 16], [16], [31, 32], [32], [63, 64], [64], [127, 128], [128], [250, 253],
+                                  [0, 1, 2, 4, 8, 16, 32, 64, 128], [15, 16, 31, 48, 80, 96, 112, 144, 176, 208, 240]])
+def test_doubling_chains(gpu, oracle, bits):
+    """Few finite results, at the edges of the tree's levels (four lanes per
+    doubling below 16 bits, a warp per point from there): chains of every
+    length, with and without an addition at their end; exact arithmetic."""
+    table = H.load_g_bases()
+    rng = np.random.Generator(np.random.PCG64(sum(bits)))
+    pts = {i: table[int(rng.integers(0, 256))] for i in bits}
+    zs = [int.from_bytes(rng.bytes(32), "little") % P or 1 for _ in range(254)]
+    res = results_of(pts, zs)
+    assert final_sum(gpu, res) == oracle.horner(res)
