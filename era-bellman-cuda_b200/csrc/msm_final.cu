@@ -4,35 +4,71 @@
 // reference leaves this Horner pass to its callers, on the host
 // (src/bellman-cuda.h:496-505; tests/msm_test.cu:116-126).
 //
-// Whatever the order of the additions, the term 2^253 R_253 needs 253
-// dependent doublings, so the sum is latency-bound: one block, and what counts
-// is the time of one doubling.  A Horner pass also puts 253 additions on that
-// chain; a pairwise tree over the bits puts 8: part t starts from R_2t + 2
-// R_2t+1, and at level L = 1..7 the sum starting at bit 2t (t mod 2^L = 0)
-// takes its partner's (t + 2^(L-1)), doubled 2^L times.
+// Doublings are what the sum costs: 2^253 R_253 taken plainly needs 253
+// dependent ones, whatever the order of the additions.  Here the chain is about
+// half as long, because BN254 (j = 0) has the endomorphism phi(x, y) =
+// (beta x, y) = lambda (x, y), and with it any multiple k P is a P + b phi(P)
+// for some |a|, |b| < 2^126 (R. Gallant, R. Lambert, S. Vanstone, "Faster point
+// multiplication on elliptic curves with efficient endomorphisms", CRYPTO
+// 2001).  A cluster of eight blocks works in three steps:
+//   groups   V_g = sum of 2^i R_(16 g + i) over 16 bits, two groups per block,
+//            as a pairwise tree over the bits (15 doublings, 4 additions deep)
+//   digits   2^(16 g) V_g = a_g V_g + b_g phi(V_g) for g >= 8, so the sum is
+//            that of 2^j Q_j over j < 126, Q_j adding the V_g and phi(V_g)
+//            whose a_g or b_g has bit j (and V_(j / 16) itself for j = 0, 16,
+//            ..., 112); 16 bits j per block, at most 16 terms each
+//   bits     the sum of 2^j Q_j, a pairwise tree over the bits: 16 in each
+//            block, the last three levels in the first block
+// so 15 + 127 doublings are dependent, and about 12 additions between them.
 //
-// Levels 0 to 2 (many points, few doublings) share each doubling between four
-// lanes (dbl_group4).  From level 3 on a warp takes one point and doubles it in
-// a residue number system (rns.cuh), where a product of the whole warp takes
+// Levels of one or two doublings share each one between four lanes
+// (dbl_group4).  The others give a warp to each point and double it in a
+// residue number system (rns.cuh), where a product of the whole warp takes
 // less than half of one thread's: about 1,030 cycles per doubling on a B200
-// against 3,236 for dbl_group4; one final sum 0.544 -> 0.230 ms, of a batched
-// instance's results (20 bits) 0.083 ms.
-// The affine conversion takes one inversion (inverse_group4).
+// against 3,236 for dbl_group4.  The affine conversion takes one inversion
+// (inverse_group4).
+// One final sum takes 0.172 ms on a B200 (0.230 ms in one block without phi,
+// the 253 doublings one after another; 0.189 ms with the steps' code repeated),
+// of a batched instance's results (20 bits) 0.072 ms.
 #include "bellman-cuda-b200.h"
 #include "msm_device.cuh"
 #include "msm_group4.cuh"
 #include "pointer_access.h"
 #include "rns.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 namespace msm_b200 {
 
-constexpr unsigned FINAL_PARTS = 128; // parts t < 127 start from results 2t, 2t + 1
-constexpr unsigned FINAL_THREADS = 4 * FINAL_PARTS;
-constexpr unsigned FINAL_WARPS = FINAL_THREADS / 32;
-constexpr unsigned FINAL_RNS_LEVEL = 3; // the first level with a warp per point
-static_assert(FINAL_PARTS >> FINAL_RNS_LEVEL <= FINAL_WARPS, "a warp per point");
+constexpr unsigned FINAL_BLOCKS = 8; // one cluster
+constexpr unsigned FINAL_PARTS = 16; // per block: pairs of results, then bits of the sum
+constexpr unsigned FINAL_THREADS = 256, FINAL_WARPS = FINAL_THREADS / 32;
+constexpr unsigned FINAL_RNS_DOUBLINGS = 4; // levels of at least this many doublings take a warp per point
+constexpr unsigned GROUP_BITS = 16, GROUPS = FINAL_BLOCKS * 2, SPLIT_GROUPS = GROUPS / 2; // groups g >= SPLIT_GROUPS are split by phi
+static_assert(FINAL_BLOCKS * FINAL_PARTS * 2 >= RESULT_BITS && GROUPS * GROUP_BITS >= RESULT_BITS, "all results");
+
+// 2^(16 g) = (-1)^a_negative a + (-1)^b_negative b lambda modulo the group
+// order for g = 8..15, lambda = 0xb3c4d79d41a917585bfc41088d8daaa78b17ea66b99c90dd
+struct split_power {
+  uint32_t a[4], b[4];
+  bool a_negative, b_negative;
+};
+__device__ const split_power split_powers[SPLIT_GROUPS] = {
+    {{0xdbbdb5ea, 0xe8363d57, 0x228f4c05, 0x2164fb6e}, {0x29a427c6, 0x13a64ad1, 0x00000001, 0x00000000}, false, true},
+    {{0xc9e237e5, 0x539f4c9e, 0x75c1faee, 0x06ebdd48}, {0xdb8b788d, 0x6ba77562, 0x00013d00, 0x00000000}, true, true},
+    {{0xa24c59e7, 0xf85004a5, 0x0a6de4a2, 0x267f96d2}, {0x8c8a719f, 0x915e63d2, 0x3d006315, 0x00000001}, true, true},
+    {{0x0b0af5fc, 0xd6058217, 0xf8e2c5d6, 0x13a5b87b}, {0xd7e617dc, 0x6f7e2430, 0x631561b2, 0x00013d00}, true, true},
+    {{0x9768ca72, 0x62da6d02, 0x5343de7f, 0x3540c909}, {0xc9c5e8eb, 0xe101e709, 0x6a76b6cb, 0x10e823c5}, false, false},
+    {{0xa407db0b, 0xdb74ec20, 0x9daeb672, 0x109889d3}, {0x23f8f66c, 0x72aec238, 0x5407a725, 0x0f4befa4}, true, true},
+    {{0x22dd5037, 0xecc76690, 0xae9818db, 0x18d59a49}, {0x9d7fbb5c, 0x93928275, 0x6100ad02, 0x18668fff}, false, false},
+    {{0x4941ded8, 0x1f927622, 0xdb80324c, 0x221b5563}, {0x772a38ab, 0x2d4e87c5, 0x710052ca, 0x211ca5f3}, true, false},
+};
+
+// beta 2^256 mod p, beta = 0x59e26bcea0d48bacd4f263f1acdb5c4f5763473177fffffe
+__device__ __forceinline__ fe endomorphism_beta() {
+  return {{0xd782e155, 0x71930c11, 0xffbe3323, 0xa6bb947c, 0xd4741444, 0xaa303344, 0x26594943, 0x2c3b3f0d}};
+}
 
 __device__ const rns::tables rns_tables = rns::TABLES;
 
@@ -134,66 +170,142 @@ struct rns_warp {
   }
 };
 
-__global__ void __launch_bounds__(FINAL_THREADS) final_sum_kernel(const jacobian *__restrict__ results, msm_b200_affine_point *point) {
-  __shared__ xyzz part[FINAL_PARTS]; // part[t]: the sum of the bits starting at 2t (weights relative to 2^2t)
-  __shared__ int64_t columns[FINAL_WARPS][rns::GROUPS][8];
-  const unsigned t = threadIdx.x, group = t >> 2, role = t & 3, warp = t >> 5;
-  { // level 0, four lanes per pair of results
-    const unsigned lane_base = t & 28;
-    jacobian lo, hi;
-    lo.x = lo.y = lo.z = hi.x = hi.y = hi.z = fq::zero();
-    if (2 * group + 1 < RESULT_BITS) {
-      lo = results[2 * group];
-      hi = results[2 * group + 1];
-    }
-    const fe z = select_fe(role & 1, hi.z, lo.z); // Z^2 and Z^3 of both points, one per lane
-    const fe zz = fq::sqr(z), zzz = fq::mul(zz, z);
-    const xyzz a = {lo.x, lo.y, shfl_fe(zz, lane_base), shfl_fe(zzz, lane_base)};
-    const xyzz b = {hi.x, hi.y, shfl_fe(zz, lane_base + 1), shfl_fe(zzz, lane_base + 1)};
-    const xyzz q = add_group4(a, dbl_group4(b));
-    if (role == 0)
-      part[group] = q;
-  }
-  __syncthreads();
-  // levels 1 and 2: group g of four lanes adds part[g 2^L + 2^(L-1)], doubled
-  // 2^L times, into part[g 2^L] (whole warps: 64 and 32 groups)
-  for (unsigned level = 1; level < FINAL_RNS_LEVEL; level++) {
-    if (group < FINAL_PARTS >> level) {
-      const unsigned target = group << level;
-      xyzz o = part[target + (1u << (level - 1))];
-      if (!__all_sync(0xffffffffu, curve::is_inf(o)))
-        for (unsigned k = 0; k < (1u << level); k++)
-          o = dbl_group4(o);
-      const xyzz q = add_group4(part[target], o);
-      __syncwarp();
-      if (role == 0)
-        part[target] = q;
-    }
-    __syncthreads();
-  }
-  // the other levels, a warp per point; an infinite partner adds nothing (the
-  // batched path's results are infinity above bit c - 1)
-  const rns_warp w;
-  for (unsigned level = FINAL_RNS_LEVEL; (1u << level) <= FINAL_PARTS; level++) {
-    if (warp < FINAL_PARTS >> level) {
-      const unsigned target = warp << level, partner = target + (1u << (level - 1));
-      if (!curve::is_inf(part[partner])) {
-        rns_point o = w.load(part[partner]);
-        for (unsigned k = 0; k < (1u << level); k++)
-          o = w.doubled(o);
-        const jacobian j = w.store(o, columns[warp]);
-        const xyzz q = add_group4(part[target], curve::from_jacobian(j));
-        __syncwarp();
-        if ((t & 31) == 0)
-          part[target] = q;
+struct final_shared {
+  xyzz part[FINAL_PARTS];
+  xyzz group[GROUPS];            // every block's two group sums
+  xyzz choice[SPLIT_GROUPS][3];  // of a split group, signed: V, phi(V), their sum
+  int64_t columns[FINAL_WARPS][rns::GROUPS][8];
+};
+
+// copies one XYZZ point from block `rank`'s shared memory (8 lanes)
+__device__ __forceinline__ void copy_remote(cooperative_groups::cluster_group &cluster, xyzz *to, xyzz *from, unsigned rank, unsigned lane8) {
+  reinterpret_cast<uint4 *>(to)[lane8] = reinterpret_cast<const uint4 *>(cluster.map_shared_rank(from, rank))[lane8];
+}
+
+// The digits step: part[b] = Q_(16 rank + b) from sh.group.  Sixteen lanes per
+// bit, four per share; share s takes the split groups 2 s and 2 s + 1.
+__device__ __forceinline__ void sum_digits(final_shared &sh, unsigned rank) {
+  const unsigned t = threadIdx.x, j = rank * FINAL_PARTS + (t >> 4), share = (t >> 2) & 3;
+  auto chosen = [&](unsigned g) {
+    const split_power &power = split_powers[g];
+    const unsigned a = (power.a[j >> 5] >> (j & 31)) & 1, b = (power.b[j >> 5] >> (j & 31)) & 1;
+    return a + b ? sh.choice[g][a + 2 * b - 1] : curve::infinity();
+  };
+  xyzz acc = curve::infinity(), p = curve::infinity();
+  // every addition of the step through one place: the code is too large to
+  // repeat (each copy is fetched once per call)
+#pragma unroll 1
+  for (unsigned pass = 0; pass < 5; pass++) {
+    const bool first_warp = t < 32, run = first_warp || (pass != 0 && pass != 4);
+    if (pass == 0) {
+      if (first_warp) {
+        const unsigned g = t >> 2;
+        acc = sh.group[SPLIT_GROUPS + g];
+        p = acc;
+        p.x = fq::mul(p.x, endomorphism_beta());
+        acc.y = select_fe(split_powers[g].a_negative, fq::neg(acc.y), acc.y);
+        p.y = select_fe(split_powers[g].b_negative, fq::neg(p.y), p.y);
+        if ((t & 3) == 0) {
+          sh.choice[g][0] = acc;
+          sh.choice[g][1] = p;
+        }
       }
+    } else if (pass == 1) {
+      acc = chosen(2 * share);
+      p = chosen(2 * share + 1);
+    } else if (pass < 4) {
+      p = shfl_xyzz(acc, (t & 31) ^ (1u << pass));
+    } else { // bit 16 rank also takes the unsplit group of that weight
+      p = select_xyzz(t < 4, sh.group[rank], curve::infinity());
+    }
+    if (run && __any_sync(0xffffffffu, !curve::is_inf(p)))
+      acc = add_group4(acc, p);
+    if (pass == 0) {
+      if (first_warp && (t & 3) == 0)
+        sh.choice[t >> 2][2] = acc;
+      __syncthreads();
+    }
+  }
+  if ((t & 15) == 0)
+    sh.part[t >> 4] = acc;
+  __syncthreads();
+}
+
+__global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THREADS)
+    final_sum_kernel(const jacobian *__restrict__ results, msm_b200_affine_point *point) {
+  __shared__ final_shared sh;
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const unsigned t = threadIdx.x, role = t & 3, rank = cluster.block_rank();
+  const rns_warp w;
+  // One tree level per step: part[g 2^L] += 2^n part[g 2^L + 2^(L-1)].  Step 0
+  // forms the pairs R_2p + 2 R_2p+1; steps 1..3 are the groups' levels, 4..7
+  // the bits' levels, 8..10 the last three in block 0.  One loop, so that every
+  // step runs the same code (copies per step cost an instruction fetch each).
+#pragma unroll 1
+  for (unsigned step = 0; step < 11; step++) {
+    if (step == 4) {
+      cluster.sync();
+      if (t < 8 * GROUPS) // group g: part 0 or 8 of block g / 2
+        copy_remote(cluster, &sh.group[t >> 3], &sh.part[((t >> 3) & 1) * (FINAL_PARTS / 2)], t >> 4, t & 7);
+      cluster.sync(); // every block has read the parts before they change
+      sum_digits(sh, rank);
+    } else if (step == 8) {
+      cluster.sync();
+      if (rank == 0 && t >= 8 && t < 8 * FINAL_BLOCKS) // block k's sum, of bits from 16 k on, into part 2 k
+        copy_remote(cluster, &sh.part[2 * (t >> 3)], &sh.part[0], t >> 3, t & 7);
+      cluster.sync(); // the other blocks stay until their sums are read
+      if (rank != 0)
+        return;
+    }
+    const unsigned level = step < 4 ? step : step < 8 ? step - 3 : step - 6;
+    const unsigned n = step < 4 ? 1u << level : step < 8 ? 1u << (level - 1) : 4u << level;
+    const unsigned pairs = FINAL_PARTS >> level, half = (1u << level) >> 1;
+    const bool by_lanes = n < FINAL_RNS_DOUBLINGS; // four lanes per pair, or a warp
+    if ((by_lanes ? (t & ~31u) >> 2 : t >> 5) < pairs) { // the warp has a pair; groups of lanes without one redo the first
+      const bool active = !by_lanes || t >> 2 < pairs;
+      const unsigned pair = by_lanes ? (active ? t >> 2 : 0) : t >> 5, target = pair << level;
+      xyzz q, o;
+      if (step == 0) {
+        const unsigned r = 2 * (rank * FINAL_PARTS + pair);
+        jacobian lo, hi;
+        lo.x = lo.y = lo.z = hi.x = hi.y = hi.z = fq::zero();
+        if (r + 1 < RESULT_BITS) {
+          lo = results[r];
+          hi = results[r + 1];
+        }
+        const fe z = select_fe(role & 1, hi.z, lo.z); // Z^2 and Z^3 of both points, one per lane
+        const fe zz = fq::sqr(z), zzz = fq::mul(zz, z);
+        q = {lo.x, lo.y, shfl_fe(zz, t & 28), shfl_fe(zzz, t & 28)};
+        o = {hi.x, hi.y, shfl_fe(zz, (t & 28) + 1), shfl_fe(zzz, (t & 28) + 1)};
+      } else {
+        q = sh.part[target];
+        o = sh.part[target + half];
+      }
+      // an infinite partner adds nothing (the batched path's results are infinity above bit c - 1)
+      if (!__all_sync(0xffffffffu, curve::is_inf(o))) {
+        if (by_lanes) {
+#pragma unroll 1
+          for (unsigned k = 0; k < n; k++)
+            o = dbl_group4(o);
+        } else {
+          rns_point d = w.load(sh.part[target + half]);
+#pragma unroll 1
+          for (unsigned k = 0; k < n; k++)
+            d = w.doubled(d);
+          o = curve::from_jacobian(w.store(d, sh.columns[t >> 5]));
+        }
+        q = add_group4(q, o);
+      }
+      __syncwarp();
+      if (active && (by_lanes ? role == 0 : (t & 31) == 0))
+        sh.part[target] = q;
     }
     __syncthreads();
   }
   // affine: one inversion of ZZ ZZZ gives 1 / ZZ = ZZZ / (ZZ ZZZ) and 1 / ZZZ;
   // lane 0 finishes x, lane 1 y
   if (t < 32) {
-    const xyzz p = part[0];
+    const xyzz p = sh.part[0];
     const fe inverse = fq::to_mont(inverse_group4(fq::from_mont(fq::mul(p.zz, p.zzz))));
     const bool is_x = t == 0, infinity = curve::is_inf(p);
     const fe c = fq::from_mont(fq::mul(select_fe(is_x, p.x, p.y), fq::mul(select_fe(is_x, p.zzz, p.zz), inverse)));
@@ -232,7 +344,7 @@ cudaError_t final_sum(const void *results, msm_b200_affine_point *point, cudaStr
     err = device_view(point, &p);
   if (err != cudaSuccess)
     return err;
-  final_sum_kernel<<<1, FINAL_THREADS, 0, stream>>>(static_cast<const jacobian *>(r), static_cast<msm_b200_affine_point *>(p));
+  final_sum_kernel<<<FINAL_BLOCKS, FINAL_THREADS, 0, stream>>>(static_cast<const jacobian *>(r), static_cast<msm_b200_affine_point *>(p));
   return cudaGetLastError();
 }
 
