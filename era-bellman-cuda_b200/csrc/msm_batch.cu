@@ -30,6 +30,7 @@
 #include "msm_device.cuh"
 #include "msm_batch.cuh"
 #include "msm_host.cuh"
+#include "msm_reduce.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -296,30 +297,30 @@ __global__ void __launch_bounds__(ACC_THREADS, ACC_MIN_BLOCKS) batch_accumulate_
 
 // Results of the instances of one reduction group (all of window width c):
 // instance members[w] is window w of the group's reduction.  Bit i < c comes
-// from the group's streams exactly as gather_results_kernel places window 0
-// of a plain MSM; bits >= c are infinity.
-__global__ void batch_gather_kernel(const xyzz *__restrict__ streams, const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
-                                    const unsigned *__restrict__ members, unsigned windows, unsigned c, unsigned log_m, unsigned log_g,
-                                    const batch_io *__restrict__ io) {
-  const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= windows * RESULT_BITS)
-    return;
-  const unsigned w = gid / RESULT_BITS, i = gid % RESULT_BITS;
-  xyzz p = curve::infinity();
-  if (i < c) {
-    const size_t base = (size_t)w * stream_stride(log_g);
+// from the group's streams exactly as reduce_tail_kernel places window 0 of a
+// plain MSM; bits >= c are infinity.
+__global__ void __launch_bounds__(TAIL_THREADS) batch_reduce_tail_kernel(const xyzz *__restrict__ tree, const xyzz *__restrict__ streams,
+                                                                         const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
+                                                                         const unsigned *__restrict__ members, unsigned c, unsigned log_m,
+                                                                         unsigned log_g, unsigned level, const batch_io *__restrict__ io) {
+  const unsigned w = blockIdx.x, i = threadIdx.x;
+  reduce_tail(tree, streams, w, log_g, level, [&](auto sum) {
+    if (i >= RESULT_BITS)
+      return;
+    xyzz p = curve::infinity();
     if (i == 0) {
-      p = load_xyzz(streams + base);
+      p = sum(0);
     } else if (i == c - 1) {
       const size_t slot0 = (size_t)w << (c - 1);
       if (flags[slot0])
         p = load_xyzz(buckets + slot0);
-    } else if (i >= log_m && i - log_m < log_g) {
-      p = load_xyzz(streams + base + stream_offset(log_g, i - log_m + 1));
+    } else if (i < c && i >= log_m && i - log_m < log_g) {
+      p = sum(i - log_m + 1);
     }
-  }
-  store_jacobian(io[members[w]].results + i, curve::to_jacobian(p));
+    store_jacobian(io[members[w]].results + i, curve::to_jacobian(p));
+  });
 }
+static_assert(TAIL_THREADS >= RESULT_BITS, "a thread per result");
 
 // ---------------------------------------------------------------------------
 // host side
@@ -697,10 +698,10 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
     xyzz *const tree[2] = {reinterpret_cast<xyzz *>(at(grp.tree[0])), reinterpret_cast<xyzz *>(at(grp.tree[1]))};
     xyzz *const streams[2] = {reinterpret_cast<xyzz *>(at(grp.streams[0])), reinterpret_cast<xyzz *>(at(grp.streams[1]))};
     CHECK(enqueue_window_sums(p, gb, gf, tree, streams, fs, launched));
-    const int si = p.log_g & 1;
-    const unsigned gather_threads = p.windows * RESULT_BITS;
-    batch_gather_kernel<<<(gather_threads + 127) / 128, 128, 0, fs>>>(streams[si], gb, gf, reinterpret_cast<const unsigned *>(at(grp.members_dev)),
-                                                                      p.windows, p.c, p.log_m, p.log_g, io);
+    const unsigned level = tail_level(p.log_g);
+    batch_reduce_tail_kernel<<<p.windows, TAIL_THREADS, tail_smem(p.log_g), fs>>>(tree[level & 1], streams[level & 1], gb, gf,
+                                                                                  reinterpret_cast<const unsigned *>(at(grp.members_dev)), p.c,
+                                                                                  p.log_m, p.log_g, level, io);
     CHECK(cudaGetLastError());
     launched++;
     if (forks) {

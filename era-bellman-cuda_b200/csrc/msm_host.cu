@@ -582,7 +582,8 @@ cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsign
   return cudaSuccess;
 }
 
-// Stage 6: bucket reduction of (buckets, flags) into the 254 results.  Blocks
+// Stage 6: bucket reduction of (buckets, flags) up to level tail_level(log_g),
+// from where reduce_tail_kernel finishes it.  Blocks
 // of ACC_THREADS: at 2^22, blocks of 64 threads measured the same and blocks
 // of 96 slower (reduction 0.695 -> 0.815 ms).
 cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_t *flags, xyzz *const tree[2], xyzz *const streams[2],
@@ -600,7 +601,7 @@ cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_
     reduce_groups_kernel<<<blocks(group_threads), ACC_THREADS, 0, stream>>>(buckets, flags, p.windows, p.log_b, p.log_m, tree[0], streams[0]);
   CHECK(cudaGetLastError());
   launched++;
-  for (unsigned level = 0; level < p.log_g; level++) {
+  for (unsigned level = 0; level < tail_level(p.log_g); level++) {
     const unsigned threads = p.windows * (level + 2) * ((1u << p.log_g) >> (level + 1));
     const int in = level & 1;
     if (threads <= small)
@@ -620,8 +621,9 @@ static cudaError_t enqueue_reduction(const plan &p, const xyzz *buckets, const u
   xyzz *const tree[2] = {reinterpret_cast<xyzz *>(scratch + l.tree[0]), reinterpret_cast<xyzz *>(scratch + l.tree[1])};
   xyzz *const streams[2] = {reinterpret_cast<xyzz *>(scratch + l.streams[0]), reinterpret_cast<xyzz *>(scratch + l.streams[1])};
   CHECK(enqueue_window_sums(p, buckets, flags, tree, streams, stream, m.launched));
-  gather_results_kernel<<<(RESULT_BITS + 127) / 128, 128, 0, stream>>>(streams[p.log_g & 1], buckets, flags, p.windows, p.c, p.log_m, p.log_g,
-                                                                       results);
+  const unsigned level = tail_level(p.log_g);
+  reduce_tail_kernel<<<p.windows, TAIL_THREADS, tail_smem(p.log_g), stream>>>(tree[level & 1], streams[level & 1], buckets, flags, p.c, p.log_m,
+                                                                             p.log_g, level, results);
   CHECK(cudaGetLastError());
   m.launched++;
   CHECK(m.mark(stream));

@@ -2,6 +2,7 @@
 // overall data flow.
 #include "msm_affine.cuh"
 #include "msm_group4.cuh"
+#include "msm_reduce.cuh"
 
 namespace msm_b200 {
 
@@ -607,26 +608,25 @@ __global__ void __launch_bounds__(ACC_THREADS) reduce_level_group4_kernel(const 
 
 // Result bit i = c*w + o:  o == 0 -> stream 0;  o == c-1 -> slot 0 (|d| = B);
 // log_m <= o < c-1 -> stream o - log_m + 1;  otherwise infinity.
-__global__ void gather_results_kernel(const xyzz *__restrict__ streams, const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
-                                      unsigned windows, unsigned c, unsigned log_m, unsigned log_g, jacobian *__restrict__ results) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= RESULT_BITS)
-    return;
-  const unsigned w = i / c, o = i % c;
-  xyzz p = curve::infinity();
-  if (w < windows) {
-    const size_t base = (size_t)w * stream_stride(log_g);
+__global__ void __launch_bounds__(TAIL_THREADS) reduce_tail_kernel(const xyzz *__restrict__ tree, const xyzz *__restrict__ streams,
+                                                                   const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags, unsigned c,
+                                                                   unsigned log_m, unsigned log_g, unsigned level, jacobian *__restrict__ results) {
+  const unsigned w = blockIdx.x, o = threadIdx.x;
+  reduce_tail(tree, streams, w, log_g, level, [&](auto sum) {
+    if (o >= c || w * c + o >= RESULT_BITS)
+      return;
+    xyzz p = curve::infinity();
     if (o == 0) {
-      p = load_xyzz(streams + base + stream_offset(log_g, 0));
+      p = sum(0);
     } else if (o == c - 1) {
       const unsigned slot0 = w << (c - 1);
       if (flags[slot0])
         p = load_xyzz(buckets + slot0);
     } else if (o >= log_m && o - log_m < log_g) {
-      p = load_xyzz(streams + base + stream_offset(log_g, o - log_m + 1));
+      p = sum(o - log_m + 1);
     }
-  }
-  store_jacobian(results + i, curve::to_jacobian(p));
+    store_jacobian(results + w * c + o, curve::to_jacobian(p));
+  });
 }
 
 } // namespace msm_b200

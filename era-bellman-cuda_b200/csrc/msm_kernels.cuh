@@ -233,8 +233,37 @@ __global__ void reduce_groups_group4_kernel(const xyzz *__restrict__ buckets, co
                                             unsigned log_m, xyzz *__restrict__ run, xyzz *__restrict__ streams);
 __global__ void reduce_level_group4_kernel(const xyzz *__restrict__ t_in, xyzz *__restrict__ t_out, const xyzz *__restrict__ s_in,
                                            xyzz *__restrict__ s_out, unsigned windows, unsigned log_g, unsigned level);
-__global__ void gather_results_kernel(const xyzz *__restrict__ streams, const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
-                                      unsigned windows, unsigned c, unsigned log_m, unsigned log_g, jacobian *__restrict__ results);
+// The last levels of the reduction and the results in one launch, one block
+// per window (reduce_tail in msm_reduce.cuh): entered at level
+// tail_level(log_g), dynamic shared memory tail_smem(log_g).
+constexpr unsigned TAIL_THREADS = 256;
+__global__ void reduce_tail_kernel(const xyzz *__restrict__ tree, const xyzz *__restrict__ streams, const xyzz *__restrict__ buckets,
+                                   const uint8_t *__restrict__ flags, unsigned c, unsigned log_m, unsigned log_g, unsigned level,
+                                   jacobian *__restrict__ results);
+
+// The level from which one block per window finishes the reduction: the first
+// with at most TAIL_JOBS additions per window, one and a half rounds of the
+// block's 64 groups of four lanes.  A level's launch costs more than its one
+// dependent addition there: the MSM with a launch per level and one for the
+// results took 0.151 ms at 2^8 points (c = 5), 0.200 at 2^12 (c = 8), 0.415 at
+// 30,000 (c = 9), 1.140 at 2^18 (c = 15) and 10.840 at 2^22 (c = 17); with
+// this 0.141, 0.183, 0.403, 1.134 and 10.826.  Larger levels need the other SMs.
+constexpr unsigned TAIL_JOBS = 96;
+__host__ __device__ constexpr unsigned tail_level(unsigned log_g) {
+  unsigned level = 0;
+  while (level < log_g && (level + 2) * ((1u << (log_g - level)) / 2) > TAIL_JOBS)
+    level++;
+  return level;
+}
+// streams 0..level and the tree of E = G >> level entries, and the later
+// streams of E / 2, E / 4, ... entries
+__host__ __device__ constexpr size_t tail_smem(unsigned log_g) {
+  const unsigned level = tail_level(log_g);
+  return ((size_t)(level + 3) << (log_g - level)) * sizeof(xyzz);
+}
+static_assert(tail_smem(6) <= 48 << 10 && tail_smem(7) <= 48 << 10 && tail_smem(8) <= 48 << 10 && tail_smem(9) <= 48 << 10 &&
+                  tail_smem(14) <= 48 << 10 && tail_smem(23) <= 48 << 10,
+              "the tail needs no opt-in shared memory (7 is the largest)");
 
 // stride of the per-window plain-sum streams (stream 0: G entries, stream s: G >> s)
 __host__ __device__ __forceinline__ size_t stream_stride(unsigned log_g) { return (size_t)2 << log_g; }

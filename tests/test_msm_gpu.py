@@ -318,6 +318,23 @@ def test_any_window_and_length(gpu, oracle, window_bits):
     assert oracle.horner(res) == oracle.msm_checksum(k, scalars)
 
 
+@pytest.mark.parametrize("window_bits", [4, 6, 7, 9, 10, 12, 14, 15, 18, 19])
+def test_reduction_tails(gpu, oracle, window_bits):
+    """The widths test_any_window_and_length leaves out: the reduction's last
+    levels run in one block per window from level 0 (c <= 8), 1 (c = 9) up to
+    15 (c = 19), exact against the oracle."""
+    n = 1777
+    bases, scalars, k = H.table_workload(n, 820 + window_bits)
+    bd, sd = gpu.upload(bases), gpu.upload(scalars)
+    rd = gpu.bc.malloc(254 * 96)
+    assert gpu.bc.msm_any(gpu.pool, gpu.stream, bd, sd, rd, n, window_bits) == 0
+    gpu.bc.stream_synchronize(gpu.stream)
+    res = gpu.bc.from_device(rd, (254, 24))
+    for p in (bd, sd, rd):
+        gpu.bc.free(p)
+    assert oracle.horner(res) == oracle.msm_checksum(k, scalars)
+
+
 @pytest.mark.parametrize("n,window_bits", [(4097, 13), (8191, 15), (12289, 16), (65537, 17), (200003, 17), (131071, 9)])
 def test_sort_tile_edges(gpu, oracle, n, window_bits):
     """Lengths just past and short of whole sort tiles (4096 keys), skewed
