@@ -382,31 +382,47 @@ __global__ void __launch_bounds__(ACC_THREADS) merge_heads_kernel(const uint32_t
   const unsigned long long k = (unsigned long long)w * 32 + lane;
   const uint32_t b = k < n_in ? hb_in[k] : INVALID_BUCKET;
   xyzz acc = b != INVALID_BUCKET ? load_xyzz(hp_in + k) : curve::infinity();
-#pragma unroll
-  for (unsigned d = 1; d < 32; d <<= 1) {
-    const uint32_t bo = __shfl_up_sync(0xffffffffu, b, d);
-    const xyzz o = shfl_up_xyzz(acc, d);
-    if (lane >= d && bo == b && b != INVALID_BUCKET)
+  bool owner = false; // this lane's sum goes into its bucket
+  unsigned first = 0;
+  bool continued = false;
+  // The scan's five steps, then the bucket additions, through one addition:
+  // each copy of it is some 2,000 instructions, and a launch of a few dependent
+  // steps mostly waits for its code.  Six copies here, four in
+  // merge_heads_group4_kernel and three in the group sums against one each: MSM at
+  // 2^12 points 0.183 -> 0.171 ms, 30,000 0.403 -> 0.385, 200,003 skewed 0.672
+  // -> 0.582, 2^18 1.134 -> 1.110, 2^22 skewed 3.768 -> 3.670.
+#pragma unroll 1
+  for (unsigned d = 1; d <= 32; d <<= 1) {
+    xyzz o;
+    bool take;
+    if (d < 32) {
+      const uint32_t bo = __shfl_up_sync(0xffffffffu, b, d);
+      o = shfl_up_xyzz(acc, d);
+      take = lane >= d && bo == b && b != INVALID_BUCKET;
+    } else {
+      const uint32_t prev = __shfl_up_sync(0xffffffffu, b, 1), next = __shfl_down_sync(0xffffffffu, b, 1);
+      const unsigned joins = __ballot_sync(0xffffffffu, lane > 0 && prev == b); // lane continues lane - 1's segment
+      first = 31 - __clz(~joins & ((2u << lane) - 1));                        // first lane of this lane's segment
+      const uint32_t b0 = __shfl_sync(0xffffffffu, b, 0);
+      uint32_t before = INVALID_BUCKET;
+      if (lane == 0 && w > 0)
+        before = hb_in[(size_t)w * 32 - 1];
+      before = __shfl_sync(0xffffffffu, before, 0);
+      continued = b0 != INVALID_BUCKET && before == b0; // lane 0's segment began in an earlier warp
+      const bool last = lane == 31 || next != b;
+      if (b != INVALID_BUCKET && last && first == 0 && continued) {
+        hb_out[w] = b;
+        store_xyzz(hp_out + w, acc);
+      }
+      take = owner = b != INVALID_BUCKET && last && !(first == 0 && continued);
+      if (take)
+        o = load_xyzz(buckets + b);
+    }
+    if (take)
       acc = curve::add(o, acc);
   }
-  const uint32_t prev = __shfl_up_sync(0xffffffffu, b, 1), next = __shfl_down_sync(0xffffffffu, b, 1);
-  const unsigned joins = __ballot_sync(0xffffffffu, lane > 0 && prev == b); // lane continues lane - 1's segment
-  const unsigned first = 31 - __clz(~joins & ((2u << lane) - 1));          // first lane of this lane's segment
-  const uint32_t b0 = __shfl_sync(0xffffffffu, b, 0);
-  uint32_t before = INVALID_BUCKET;
-  if (lane == 0 && w > 0)
-    before = hb_in[(size_t)w * 32 - 1];
-  before = __shfl_sync(0xffffffffu, before, 0);
-  const bool continued = b0 != INVALID_BUCKET && before == b0; // lane 0's segment began in an earlier warp
-  const bool last = lane == 31 || next != b;
-  if (b != INVALID_BUCKET && last) {
-    if (first == 0 && continued) {
-      hb_out[w] = b;
-      store_xyzz(hp_out + w, acc);
-    } else {
-      store_xyzz(buckets + b, curve::add(load_xyzz(buckets + b), acc));
-    }
-  }
+  if (owner)
+    store_xyzz(buckets + b, acc);
   if (lane == 0 && !continued)
     hb_out[w] = INVALID_BUCKET;
 }
@@ -426,40 +442,44 @@ __global__ void __launch_bounds__(ACC_THREADS) merge_heads_group4_kernel(const u
   const unsigned long long k = (unsigned long long)w * GROUPS + g;
   const uint32_t b = k < n_in ? hb_in[k] : INVALID_BUCKET;
   xyzz acc = b != INVALID_BUCKET ? load_xyzz(hp_in + k) : curve::infinity();
+  bool continued = false, into_bucket = false;
+  // scan steps, then the bucket additions, through one addition (see above)
+#pragma unroll 1
+  for (unsigned d = 1; d <= GROUPS; d <<= 1) {
+    xyzz o;
+    bool take;
+    if (d < GROUPS) {
+      const uint32_t bo = __shfl_up_sync(0xffffffffu, b, 4 * d);
+      o = shfl_up_xyzz(acc, 4 * d);
+      take = g >= d && bo == b && b != INVALID_BUCKET;
+    } else {
+      const uint32_t prev = __shfl_up_sync(0xffffffffu, b, 4), next = __shfl_down_sync(0xffffffffu, b, 4);
+      const unsigned join_lanes = __ballot_sync(0xffffffffu, g > 0 && prev == b); // group g continues group g - 1's segment
+      unsigned joins = 0;
 #pragma unroll
-  for (unsigned d = 1; d < GROUPS; d <<= 1) {
-    const uint32_t bo = __shfl_up_sync(0xffffffffu, b, 4 * d);
-    const xyzz o = shfl_up_xyzz(acc, 4 * d);
-    const bool take = g >= d && bo == b && b != INVALID_BUCKET;
+      for (unsigned f = 0; f < GROUPS; f++)
+        joins |= ((join_lanes >> (4 * f)) & 1u) << f;
+      const unsigned first = 31 - __clz(~joins & ((2u << g) - 1)); // first group of this group's segment
+      const uint32_t b0 = __shfl_sync(0xffffffffu, b, 0);
+      uint32_t before = INVALID_BUCKET;
+      if (lane == 0 && w > 0)
+        before = hb_in[(size_t)w * GROUPS - 1];
+      before = __shfl_sync(0xffffffffu, before, 0);
+      continued = b0 != INVALID_BUCKET && before == b0; // group 0's segment began in an earlier warp
+      const bool ends = b != INVALID_BUCKET && (g == GROUPS - 1 || next != b);
+      const bool out_head = ends && first == 0 && continued;
+      if (out_head && role == 0) {
+        hb_out[w] = b;
+        store_xyzz(hp_out + w, acc);
+      }
+      take = into_bucket = ends && !out_head;
+      o = into_bucket ? load_xyzz(buckets + b) : curve::infinity();
+    }
     if (__any_sync(0xffffffffu, take))
       acc = select_xyzz(take, add_group4(o, acc), acc);
   }
-  const uint32_t prev = __shfl_up_sync(0xffffffffu, b, 4), next = __shfl_down_sync(0xffffffffu, b, 4);
-  const unsigned join_lanes = __ballot_sync(0xffffffffu, g > 0 && prev == b); // group g continues group g - 1's segment
-  unsigned joins = 0;
-#pragma unroll
-  for (unsigned f = 0; f < GROUPS; f++)
-    joins |= ((join_lanes >> (4 * f)) & 1u) << f;
-  const unsigned first = 31 - __clz(~joins & ((2u << g) - 1)); // first group of this group's segment
-  const uint32_t b0 = __shfl_sync(0xffffffffu, b, 0);
-  uint32_t before = INVALID_BUCKET;
-  if (lane == 0 && w > 0)
-    before = hb_in[(size_t)w * GROUPS - 1];
-  before = __shfl_sync(0xffffffffu, before, 0);
-  const bool continued = b0 != INVALID_BUCKET && before == b0; // group 0's segment began in an earlier warp
-  const bool ends = b != INVALID_BUCKET && (g == GROUPS - 1 || next != b);
-  const bool out_head = ends && first == 0 && continued;
-  const bool into_bucket = ends && !out_head;
-  const xyzz held = into_bucket ? load_xyzz(buckets + b) : curve::infinity();
-  if (__any_sync(0xffffffffu, into_bucket)) {
-    const xyzz sum = add_group4(held, acc);
-    if (into_bucket && role == 0)
-      store_xyzz(buckets + b, sum);
-  }
-  if (out_head && role == 0) {
-    hb_out[w] = b;
-    store_xyzz(hp_out + w, acc);
-  }
+  if (into_bucket && role == 0)
+    store_xyzz(buckets + b, acc);
   if (lane == 0 && !continued)
     hb_out[w] = INVALID_BUCKET;
 }
@@ -495,13 +515,22 @@ __global__ void __launch_bounds__(ACC_THREADS, REDUCE_GROUPS_MIN_BLOCKS) reduce_
   const unsigned w = gid >> log_g, g = gid & ((1u << log_g) - 1);
   const unsigned base = (w << log_b) + (g << log_m);
   xyzz run = curve::infinity(), acc = curve::infinity();
-  for (unsigned i = (1u << log_m) - 1; i >= 1; i--) {
-    if (flags[base + i])
-      run = curve::add(run, load_xyzz(buckets + base + i));
-    acc = curve::add(acc, run);
+  // run += X_i, acc += run for i = m - 1 .. 1, then run += X_0 (not for group
+  // 0, whose slot 0 has another weight), through one addition
+#pragma unroll 1
+  for (unsigned step = 0; step + 1 < 2u << log_m; step++) {
+    const unsigned i = (1u << log_m) - 1 - step / 2;
+    const bool into_run = (step & 1) == 0;
+    xyzz x = run;
+    if (into_run) {
+      if (!flags[base + i] || (i == 0 && g == 0))
+        continue;
+      x = load_xyzz(buckets + base + i);
+    }
+    const xyzz sum = curve::add(select_xyzz(into_run, run, acc), x);
+    run = select_xyzz(into_run, sum, run);
+    acc = select_xyzz(into_run, acc, sum);
   }
-  if (g > 0 && flags[base])
-    run = curve::add(run, load_xyzz(buckets + base));
   store_xyzz(run_out + gid, run);
   store_xyzz(streams + (size_t)w * stream_stride(log_g) + stream_offset(log_g, 0) + g, acc);
 }
@@ -557,13 +586,17 @@ __global__ void __launch_bounds__(ACC_THREADS) reduce_groups_group4_kernel(const
   const unsigned w = gid >> log_g, g = gid & ((1u << log_g) - 1);
   const unsigned base = (w << log_b) + (g << log_m);
   xyzz run = curve::infinity(), acc = curve::infinity();
-  for (unsigned i = (1u << log_m) - 1; i >= 1; i--) {
-    const xyzz x = flags[base + i] ? load_xyzz(buckets + base + i) : curve::infinity();
-    run = add_group4(run, x);
-    acc = add_group4(acc, run);
+#pragma unroll 1
+  for (unsigned step = 0; step + 1 < 2u << log_m; step++) { // as above
+    const unsigned i = (1u << log_m) - 1 - step / 2;
+    const bool into_run = (step & 1) == 0;
+    xyzz x = run;
+    if (into_run)
+      x = flags[base + i] && !(i == 0 && g == 0) ? load_xyzz(buckets + base + i) : curve::infinity();
+    const xyzz sum = add_group4(select_xyzz(into_run, run, acc), x);
+    run = select_xyzz(into_run, sum, run);
+    acc = select_xyzz(into_run, acc, sum);
   }
-  const xyzz x0 = g > 0 && flags[base] ? load_xyzz(buckets + base) : curve::infinity();
-  run = add_group4(run, x0);
   if (active && role == 0) {
     store_xyzz(run_out + gid, run);
     store_xyzz(streams + (size_t)w * stream_stride(log_g) + stream_offset(log_g, 0) + g, acc);
