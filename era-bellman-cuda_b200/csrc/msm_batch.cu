@@ -684,7 +684,7 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
       keys[cur], vals[cur], inst, b.instances, zeros, b.acc_ranges, work, buckets, flags, hb[0], hp[0]);
   CHECK(cudaGetLastError());
   launched++;
-  CHECK(enqueue_merge_heads(hb, hp, b.acc_ranges, buckets, b.sms, s, launched));
+  CHECK(enqueue_merge_heads(hb, hp, b.acc_ranges, buckets, b.sms, false, s, launched));
   if (forks)
     CHECK(cudaEventRecord(fork_events[0], s));
   for (size_t g = 0; g < b.groups.size(); g++) {

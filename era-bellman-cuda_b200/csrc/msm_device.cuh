@@ -8,6 +8,11 @@
 
 namespace msm_b200 {
 
+// First statement of every kernel that launch_after (msm_host.cuh) may launch
+// before the stream's previous kernel has ended: waits until everything that
+// kernel wrote can be read and everything it read may be overwritten.
+__device__ __forceinline__ void begin_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // 128-bit vector memory helpers
 // ---------------------------------------------------------------------------

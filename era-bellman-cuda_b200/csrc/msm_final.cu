@@ -33,6 +33,7 @@
 #include "bellman-cuda-b200.h"
 #include "msm_device.cuh"
 #include "msm_group4.cuh"
+#include "msm_host.cuh"
 #include "pointer_access.h"
 #include "rns.cuh"
 
@@ -233,6 +234,7 @@ __device__ __forceinline__ void sum_digits(final_shared &sh, unsigned rank) {
 
 __global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THREADS)
     final_sum_kernel(const jacobian *__restrict__ results, msm_b200_affine_point *point) {
+  begin_after_previous();
   __shared__ final_shared sh;
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const unsigned t = threadIdx.x, role = t & 3, rank = cluster.block_rank();
@@ -344,8 +346,8 @@ cudaError_t final_sum(const void *results, msm_b200_affine_point *point, cudaStr
     err = device_view(point, &p);
   if (err != cudaSuccess)
     return err;
-  final_sum_kernel<<<FINAL_BLOCKS, FINAL_THREADS, 0, stream>>>(static_cast<const jacobian *>(r), static_cast<msm_b200_affine_point *>(p));
-  return cudaGetLastError();
+  return launch_after(early_launches(stream), final_sum_kernel, FINAL_BLOCKS, FINAL_THREADS, 0, stream, static_cast<const jacobian *>(r),
+                      static_cast<msm_b200_affine_point *>(p));
 }
 
 } // namespace msm_b200

@@ -300,17 +300,19 @@ static layout make_layout(const plan &p, bool copy_scalars, bool copy_bases, boo
   }
   // the first pass's digit counts per (window, digit, tile); then one region
   // cleared per chunk: digit totals per (pass, window, digit), zero digits
-  // per window, a tile counter per pass, the look-back error word, and the
+  // per window, a tile counter per pass, the look-back error word, the
+  // accumulation's work counter, and the
   // look-back words of the passes after the first, per (window, look-back
   // tile, digit)
   const size_t lookback_words = (size_t)p.windows * p.lookback_tiles * SORT_RADIX;
   l.counts = take((size_t)p.windows * SORT_RADIX * p.tiles * 4);
-  l.sort_clear_bytes = ((size_t)p.sort_passes * p.windows * SORT_RADIX + p.windows + p.sort_passes + 1 + (p.sort_passes - 1) * lookback_words) * 4;
+  l.sort_clear_bytes = ((size_t)p.sort_passes * p.windows * SORT_RADIX + p.windows + p.sort_passes + 2 + (p.sort_passes - 1) * lookback_words) * 4;
   l.totals = take(l.sort_clear_bytes);
   l.zeros = l.totals + (size_t)p.sort_passes * p.windows * SORT_RADIX * 4;
   l.sort_ctrs = l.zeros + (size_t)p.windows * 4;
   l.sort_error = l.sort_ctrs + (size_t)p.sort_passes * 4;
-  l.lookback_words = l.sort_error + 4;
+  l.work = l.sort_error + 4;
+  l.lookback_words = l.work + 4;
   const size_t slots = (size_t)p.windows << p.log_b;
   l.buckets = take(slots * sizeof(xyzz));
   l.flags = take(slots);
@@ -341,7 +343,6 @@ static layout make_layout(const plan &p, bool copy_scalars, bool copy_bases, boo
     l.level_base = take(warps * 8);
     l.level_counts = take((MAX_AFFINE_LEVELS + 1) * 8);
   }
-  l.work = take(sizeof(unsigned));
   for (int i = 0; i < 2; i++) {
     l.tree[i] = take(((size_t)p.windows << p.log_g) * sizeof(xyzz));
     l.streams[i] = take((size_t)p.windows * stream_stride(p.log_g) * sizeof(xyzz));
@@ -433,36 +434,32 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
   int cur = 0;
   if (p.windows <= MAX_FUSED_HISTOGRAM_WINDOWS && p.tiles >= FUSED_DIGITS_MIN_TILES) {
     // 1. digits, with every pass's digit counts per tile
-    digits_histogram_kernel<<<p.tiles, SORT_THREADS, digit_histogram_smem(p.windows, p.sort_passes), stream>>>(
-        scalars, n, p.c, p.windows, p.sort_passes, p.tiles, keys[0], vals[0], counts, totals, zeros);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(p.early, digits_histogram_kernel, p.tiles, SORT_THREADS, digit_histogram_smem(p.windows, p.sort_passes), stream, scalars, n,
+                       p.c, p.windows, p.sort_passes, p.tiles, keys[0], vals[0], counts, totals, zeros));
     m.launched++;
     CHECK(m.mark(stream));
     // 2. sort: one scan for the first pass's tile offsets and digit totals,
     // the first pass (drops zero digits), then one look-back kernel per later
     // 8-bit pass (their digit totals come from the digit kernel)
     const unsigned prefix_rows = p.windows * SORT_RADIX;
-    sort_scan_kernel<<<(prefix_rows * 32 + 255) / 256, 256, 0, stream>>>(counts, p.tiles, prefix_rows, totals);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(p.early, sort_scan_kernel, (prefix_rows * 32 + 255) / 256, 256, 0, stream, counts, p.tiles, prefix_rows, totals));
     const dim3 grid(p.tiles, p.windows);
-    sort_scatter_first_kernel<<<grid, SORT_THREADS, 0, stream>>>(keys[0], vals[0], keys[1], vals[1], n, p.tiles, 0, counts, totals, zeros);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(p.early, sort_scatter_first_kernel, grid, SORT_THREADS, 0, stream, keys[0], vals[0], keys[1], vals[1], n, p.tiles, 0, counts,
+                       totals, zeros));
     m.launched += 2;
     cur = 1;
     uint32_t *words = reinterpret_cast<uint32_t *>(scratch + l.lookback_words);
     for (unsigned pass = 1; pass < p.sort_passes; pass++) {
-      lookback_stable_kernel<<<p.windows * p.lookback_tiles, LOOKBACK_THREADS, lookback_smem_bytes<LOOKBACK_THREADS, LOOKBACK_ITEMS>(), stream>>>(
-          keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, p.windows, p.lookback_tiles, pass * SORT_RADIX_BITS,
-          words + (size_t)(pass - 1) * p.windows * p.lookback_tiles * SORT_RADIX, totals + (size_t)pass * prefix_rows, zeros, sort_ctrs + pass,
-          sort_error);
-      CHECK(cudaGetLastError());
+      CHECK(launch_after(p.early, lookback_stable_kernel, p.windows * p.lookback_tiles, LOOKBACK_THREADS,
+                         lookback_smem_bytes<LOOKBACK_THREADS, LOOKBACK_ITEMS>(), stream, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
+                         p.windows, p.lookback_tiles, pass * SORT_RADIX_BITS, words + (size_t)(pass - 1) * p.windows * p.lookback_tiles * SORT_RADIX,
+                         totals + (size_t)pass * prefix_rows, zeros, sort_ctrs + pass, sort_error));
       m.launched++;
       cur ^= 1;
     }
   } else {
     // 1. digits (c <= 5: more windows than the digit kernel can count)
-    digits_kernel<<<(n + 255) / 256, 256, 0, stream>>>(scalars, n, p.c, p.windows, keys[0], vals[0]);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(p.early, digits_kernel, (n + 255) / 256, 256, 0, stream, scalars, n, p.c, p.windows, keys[0], vals[0]));
     m.launched++;
     CHECK(m.mark(stream));
     // 2. sort, 8 bits per pass: histogram, scan and scatter kernels
@@ -471,19 +468,16 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
       const unsigned shift = pass * SORT_RADIX_BITS;
       const dim3 grid(p.tiles, p.windows);
       if (pass == 0)
-        sort_histogram_first_kernel<<<grid, SORT_THREADS, 0, stream>>>(keys[cur], n, p.tiles, shift, counts, zeros);
+        CHECK(launch_after(p.early, sort_histogram_first_kernel, grid, SORT_THREADS, 0, stream, keys[cur], n, p.tiles, shift, counts, zeros));
       else
-        sort_histogram_kernel<<<grid, SORT_THREADS, 0, stream>>>(keys[cur], n, p.tiles, shift, counts, zeros);
-      CHECK(cudaGetLastError());
-      sort_scan_kernel<<<(rows * 32 + 255) / 256, 256, 0, stream>>>(counts, p.tiles, rows, totals);
-      CHECK(cudaGetLastError());
+        CHECK(launch_after(p.early, sort_histogram_kernel, grid, SORT_THREADS, 0, stream, keys[cur], n, p.tiles, shift, counts, zeros));
+      CHECK(launch_after(p.early, sort_scan_kernel, (rows * 32 + 255) / 256, 256, 0, stream, counts, p.tiles, rows, totals));
       if (pass == 0)
-        sort_scatter_first_kernel<<<grid, SORT_THREADS, 0, stream>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, p.tiles, shift, counts,
-                                                                     totals, zeros);
+        CHECK(launch_after(p.early, sort_scatter_first_kernel, grid, SORT_THREADS, 0, stream, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
+                           p.tiles, shift, counts, totals, zeros));
       else
-        sort_scatter_stable_kernel<<<grid, SORT_THREADS, 0, stream>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, p.tiles, shift, counts,
-                                                                      totals, zeros);
-      CHECK(cudaGetLastError());
+        CHECK(launch_after(p.early, sort_scatter_stable_kernel, grid, SORT_THREADS, 0, stream, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
+                           p.tiles, shift, counts, totals, zeros));
       m.launched += 3;
       cur ^= 1;
     }
@@ -495,7 +489,6 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
 
   // 4. accumulation: the affine pairing levels, if any, then the XYZZ pass
   unsigned *work = reinterpret_cast<unsigned *>(scratch + l.work);
-  CHECK(cudaMemsetAsync(work, 0, sizeof(unsigned), stream));
   if (p.affine_levels) {
     uint32_t *list_buckets[2] = {reinterpret_cast<uint32_t *>(scratch + l.level_buckets[0]),
                                  reinterpret_cast<uint32_t *>(scratch + l.level_buckets[1])};
@@ -538,15 +531,15 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
     accumulate_list_kernel<<<(p.tail_threads + ACC_THREADS - 1) / ACC_THREADS, ACC_THREADS, 0, stream>>>(
         list_buckets[last], list_points[last], counts_out + p.affine_levels, p.tail_ranges, work, buckets, flags, hb[0], hp[0]);
   } else {
-    accumulate_kernel<<<(p.acc_threads + ACC_THREADS - 1) / ACC_THREADS, ACC_THREADS, 0, stream>>>(
-        keys[cur], vals[cur], bases, n, p.windows, p.log_b, zeros, p.acc_ranges, work, buckets, flags, hb[0], hp[0]);
+    CHECK(launch_after(p.early, accumulate_kernel, (p.acc_threads + ACC_THREADS - 1) / ACC_THREADS, ACC_THREADS, 0, stream, keys[cur], vals[cur],
+                       bases, n, p.windows, p.log_b, zeros, p.acc_ranges, work, buckets, flags, hb[0], hp[0]));
   }
   CHECK(cudaGetLastError());
   m.launched++;
   CHECK(m.mark(stream));
 
   // 5. heads
-  CHECK(enqueue_merge_heads(hb, hp, p.tail_ranges, buckets, p.sms, stream, m.launched));
+  CHECK(enqueue_merge_heads(hb, hp, p.tail_ranges, buckets, p.sms, p.early, stream, m.launched));
   CHECK(m.mark(stream));
   return cudaSuccess;
 }
@@ -562,8 +555,8 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
 // (0.134 ms at 2^14, 0.084 at 2^22).
 constexpr unsigned MERGE_GROUP4_HEADS_PER_SM = 32;
 
-cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsigned heads, xyzz *buckets, unsigned sms, cudaStream_t stream,
-                                unsigned &launched) {
+cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsigned heads, xyzz *buckets, unsigned sms, bool early,
+                                cudaStream_t stream, unsigned &launched) {
   int h = 0;
   while (heads > 1) {
     const bool small = heads <= (unsigned long long)sms * MERGE_GROUP4_HEADS_PER_SM;
@@ -571,10 +564,9 @@ cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsign
     const unsigned out = (heads + per_warp - 1) / per_warp;
     const unsigned blocks = (unsigned)(((unsigned long long)out * 32 + ACC_THREADS - 1) / ACC_THREADS);
     if (small)
-      merge_heads_group4_kernel<<<blocks, ACC_THREADS, 0, stream>>>(hb[h], hp[h], heads, buckets, hb[h ^ 1], hp[h ^ 1]);
+      CHECK(launch_after(early, merge_heads_group4_kernel, blocks, ACC_THREADS, 0, stream, hb[h], hp[h], heads, buckets, hb[h ^ 1], hp[h ^ 1]));
     else
-      merge_heads_kernel<<<blocks, ACC_THREADS, 0, stream>>>(hb[h], hp[h], heads, buckets, hb[h ^ 1], hp[h ^ 1]);
-    CHECK(cudaGetLastError());
+      CHECK(launch_after(early, merge_heads_kernel, blocks, ACC_THREADS, 0, stream, hb[h], hp[h], heads, buckets, hb[h ^ 1], hp[h ^ 1]));
     launched++;
     heads = out;
     h ^= 1;
@@ -595,22 +587,21 @@ cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_
   auto blocks = [](unsigned long long threads) { return (unsigned)((threads + ACC_THREADS - 1) / ACC_THREADS); };
   const unsigned group_threads = p.windows << p.log_g;
   if (group_threads <= small)
-    reduce_groups_group4_kernel<<<blocks(4ull * group_threads), ACC_THREADS, 0, stream>>>(buckets, flags, p.windows, p.log_b, p.log_m, tree[0],
-                                                                                          streams[0]);
+    CHECK(launch_after(p.early, reduce_groups_group4_kernel, blocks(4ull * group_threads), ACC_THREADS, 0, stream, buckets, flags, p.windows, p.log_b,
+                       p.log_m, tree[0], streams[0]));
   else
-    reduce_groups_kernel<<<blocks(group_threads), ACC_THREADS, 0, stream>>>(buckets, flags, p.windows, p.log_b, p.log_m, tree[0], streams[0]);
-  CHECK(cudaGetLastError());
+    CHECK(launch_after(p.early, reduce_groups_kernel, blocks(group_threads), ACC_THREADS, 0, stream, buckets, flags, p.windows, p.log_b, p.log_m,
+                       tree[0], streams[0]));
   launched++;
   for (unsigned level = 0; level < tail_level(p.log_g); level++) {
     const unsigned threads = p.windows * (level + 2) * ((1u << p.log_g) >> (level + 1));
     const int in = level & 1;
     if (threads <= small)
-      reduce_level_group4_kernel<<<blocks(4ull * threads), ACC_THREADS, 0, stream>>>(tree[in], tree[in ^ 1], streams[in], streams[in ^ 1],
-                                                                                      p.windows, p.log_g, level);
+      CHECK(launch_after(p.early, reduce_level_group4_kernel, blocks(4ull * threads), ACC_THREADS, 0, stream, tree[in], tree[in ^ 1], streams[in],
+                         streams[in ^ 1], p.windows, p.log_g, level));
     else
-      reduce_level_kernel<<<blocks(threads), ACC_THREADS, 0, stream>>>(tree[in], tree[in ^ 1], streams[in], streams[in ^ 1], p.windows, p.log_g,
-                                                                       level);
-    CHECK(cudaGetLastError());
+      CHECK(launch_after(p.early, reduce_level_kernel, blocks(threads), ACC_THREADS, 0, stream, tree[in], tree[in ^ 1], streams[in], streams[in ^ 1],
+                         p.windows, p.log_g, level));
     launched++;
   }
   return cudaSuccess;
@@ -622,9 +613,8 @@ static cudaError_t enqueue_reduction(const plan &p, const xyzz *buckets, const u
   xyzz *const streams[2] = {reinterpret_cast<xyzz *>(scratch + l.streams[0]), reinterpret_cast<xyzz *>(scratch + l.streams[1])};
   CHECK(enqueue_window_sums(p, buckets, flags, tree, streams, stream, m.launched));
   const unsigned level = tail_level(p.log_g);
-  reduce_tail_kernel<<<p.windows, TAIL_THREADS, tail_smem(p.log_g), stream>>>(tree[level & 1], streams[level & 1], buckets, flags, p.c, p.log_m,
-                                                                             p.log_g, level, results);
-  CHECK(cudaGetLastError());
+  CHECK(launch_after(p.early, reduce_tail_kernel, p.windows, TAIL_THREADS, tail_smem(p.log_g), stream, tree[level & 1], streams[level & 1], buckets,
+                     flags, p.c, p.log_m, p.log_g, level, results));
   m.launched++;
   CHECK(m.mark(stream));
   return cudaSuccess;
@@ -773,7 +763,8 @@ static cudaError_t enqueue_chunked(const execution &e, const chunking &ch, const
     if (copying && j + 1 < ch.count)
       CHECK(enqueue_copy(j + 1));
     const unsigned b = ch.beg[j];
-    const plan p = make_plan(ch.size(j), full.c, sms);
+    plan p = make_plan(ch.size(j), full.c, sms);
+    p.early = full.early;
     const fe *src_scalars = copy_scalars ? scalars + ch.slot_offset(j) : static_cast<const fe *>(e.scalars) + b;
     const affine *src_bases = copy_bases ? bases + ch.slot_offset(j) : static_cast<const affine *>(e.bases) + b;
     if (copying)
@@ -783,9 +774,8 @@ static cudaError_t enqueue_chunked(const execution &e, const chunking &ch, const
     } else {
       CHECK(cudaMemsetAsync(chunk_flags, 0, slots, stream));
       CHECK(enqueue_accumulation(p, src_scalars, src_bases, chunk_buckets, chunk_flags, scratch, l, stream, m));
-      merge_chunk_buckets_kernel<<<(unsigned)((slots + ACC_THREADS - 1) / ACC_THREADS), ACC_THREADS, 0, stream>>>(buckets, flags, chunk_buckets,
-                                                                                                                 chunk_flags, (unsigned)slots);
-      CHECK(cudaGetLastError());
+      CHECK(launch_after(full.early, merge_chunk_buckets_kernel, (unsigned)((slots + ACC_THREADS - 1) / ACC_THREADS), ACC_THREADS, 0, stream, buckets,
+                         flags, chunk_buckets, chunk_flags, (unsigned)slots));
     }
     if (copying && ch.slots)
       CHECK(cudaEventRecord(r.consumed[j], stream));
@@ -827,7 +817,8 @@ cudaError_t execute(const execution &e) {
   CHECK(locate(e.results, device, &copy_results));
   const int sms = get_device_info(device).sms;
   const bool instrumented = e.profile || e.stage_events;
-  const plan p = make_plan(e.count, e.window_bits, sms);
+  plan p = make_plan(e.count, e.window_bits, sms);
+  p.early = early_launches(e.stream);
   if (p.windows > 128)
     return cudaErrorInvalidValue;
   // Memory fit (reference: the dry-run loop of msm::execute_async,
@@ -1014,6 +1005,7 @@ cudaError_t execute_no_alloc(cudaStream_t stream, const void *bases, const void 
       return cudaErrorInvalidValue;
   }
   plan p = make_plan(count, 0, get_device_info(device).sms);
+  p.early = early_launches(stream);
   set_affine_levels(p, 0);   // the fixed scratch holds no level lists
   set_reduction_groups(p, 3); // and the reduction's smallest tree (G = B / 8)
   const layout l = make_layout(p, false, false, false);

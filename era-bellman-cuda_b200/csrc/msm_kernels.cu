@@ -8,6 +8,7 @@ namespace msm_b200 {
 
 __global__ void __launch_bounds__(256) digits_kernel(const fe *__restrict__ scalars, unsigned n, unsigned c, unsigned windows,
                                                      uint32_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+  begin_after_previous();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(SORT_THREADS) digits_histogram_kernel(const fe
                                                                         unsigned passes, unsigned tiles, uint32_t *__restrict__ keys,
                                                                         uint32_t *__restrict__ vals, uint32_t *__restrict__ hist,
                                                                         uint32_t *__restrict__ totals, uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   extern __shared__ uint32_t s_hist[]; // [passes][windows][SORT_RADIX], then [windows] zero digits
   const unsigned counters = passes * windows * SORT_RADIX;
   uint32_t *zero_digits = s_hist + counters;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(LOOKBACK_THREADS, SORT_SCATTER_MIN_BLOCKS)
     lookback_stable_kernel(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, uint32_t *__restrict__ keys_out,
                            uint32_t *__restrict__ vals_out, unsigned n, unsigned windows, unsigned tiles, unsigned shift, uint32_t *words,
                            const uint32_t *__restrict__ totals, const uint32_t *__restrict__ zeros, unsigned *tile_ctr, unsigned *error) {
+  begin_after_previous();
   __shared__ unsigned s_ticket;
   if (threadIdx.x == 0)
     s_ticket = atomicAdd(tile_ctr, 1u);
@@ -139,16 +142,19 @@ __device__ __forceinline__ void sort_histogram_window(const uint32_t *__restrict
 __global__ void __launch_bounds__(SORT_THREADS) sort_histogram_first_kernel(const uint32_t *__restrict__ keys, unsigned n, unsigned tiles,
                                                                             unsigned shift, uint32_t *__restrict__ counts,
                                                                             uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   sort_histogram_window<true>(keys, n, tiles, shift, counts, zeros);
 }
 
 __global__ void __launch_bounds__(SORT_THREADS) sort_histogram_kernel(const uint32_t *__restrict__ keys, unsigned n, unsigned tiles, unsigned shift,
                                                                       uint32_t *__restrict__ counts, const uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   sort_histogram_window<false>(keys, n, tiles, shift, counts, const_cast<uint32_t *>(zeros));
 }
 
 // One warp per (window, digit) row of counts (see sort_scan_row).
 __global__ void __launch_bounds__(256) sort_scan_kernel(uint32_t *counts, unsigned tiles, unsigned rows, uint32_t *__restrict__ totals) {
+  begin_after_previous();
   const unsigned row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= rows)
     return;
@@ -160,6 +166,7 @@ __global__ void __launch_bounds__(SORT_THREADS, SORT_SCATTER_MIN_BLOCKS) sort_sc
                                                                           unsigned n, unsigned tiles, unsigned shift,
                                                                           const uint32_t *__restrict__ counts, const uint32_t *__restrict__ totals,
                                                                           const uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   const unsigned tile = blockIdx.x, w = blockIdx.y;
   const unsigned base = tile * SORT_TILE;
   const size_t seg = w * window_stride(n);
@@ -172,6 +179,7 @@ __global__ void __launch_bounds__(SORT_THREADS, SORT_SCATTER_MIN_BLOCKS) sort_sc
                                                                            unsigned n, unsigned tiles, unsigned shift,
                                                                            const uint32_t *__restrict__ counts, const uint32_t *__restrict__ totals,
                                                                            const uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   const unsigned tile = blockIdx.x, w = blockIdx.y;
   const unsigned skip = zeros[w], live = n - skip;
   const unsigned base = tile * SORT_TILE;
@@ -230,6 +238,7 @@ __global__ void __launch_bounds__(ACC_THREADS, ACC_MIN_BLOCKS) accumulate_kernel
                                                                  const uint32_t *__restrict__ zeros, unsigned ranges, unsigned *__restrict__ work,
                                                                  xyzz *__restrict__ buckets, uint8_t *__restrict__ flags,
                                                                  uint32_t *__restrict__ head_bucket, xyzz *__restrict__ head_point) {
+  begin_after_previous();
   __shared__ unsigned long long s_first[2 * MAX_WINDOWS];
   __shared__ unsigned long long s_prefix[MAX_WINDOWS + 1];
   __shared__ uint4 s_base[2][4][ACC_THREADS];
@@ -375,6 +384,7 @@ __global__ void __launch_bounds__(ACC_THREADS, ACC_MIN_BLOCKS) accumulate_list_k
 __global__ void __launch_bounds__(ACC_THREADS) merge_heads_kernel(const uint32_t *__restrict__ hb_in, const xyzz *__restrict__ hp_in,
                                                                   unsigned n_in, xyzz *__restrict__ buckets, uint32_t *__restrict__ hb_out,
                                                                   xyzz *__restrict__ hp_out) {
+  begin_after_previous();
   const unsigned lane = threadIdx.x & 31;
   const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if ((unsigned long long)w * 32 >= n_in)
@@ -434,6 +444,7 @@ __global__ void __launch_bounds__(ACC_THREADS) merge_heads_kernel(const uint32_t
 __global__ void __launch_bounds__(ACC_THREADS) merge_heads_group4_kernel(const uint32_t *__restrict__ hb_in, const xyzz *__restrict__ hp_in,
                                                                          unsigned n_in, xyzz *__restrict__ buckets, uint32_t *__restrict__ hb_out,
                                                                          xyzz *__restrict__ hp_out) {
+  begin_after_previous();
   constexpr unsigned GROUPS = MERGE_HEADS_PER_WARP_GROUP4;
   const unsigned lane = threadIdx.x & 31, g = lane >> 2, role = lane & 3;
   const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -490,6 +501,7 @@ __global__ void __launch_bounds__(ACC_THREADS) merge_heads_group4_kernel(const u
 __global__ void __launch_bounds__(ACC_THREADS) merge_chunk_buckets_kernel(xyzz *__restrict__ buckets, uint8_t *__restrict__ flags,
                                                                           const xyzz *__restrict__ chunk_buckets,
                                                                           const uint8_t *__restrict__ chunk_flags, unsigned slots) {
+  begin_after_previous();
   const unsigned b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= slots || !chunk_flags[b])
     return;
@@ -508,6 +520,7 @@ __global__ void __launch_bounds__(ACC_THREADS) merge_chunk_buckets_kernel(xyzz *
 __global__ void __launch_bounds__(ACC_THREADS, REDUCE_GROUPS_MIN_BLOCKS) reduce_groups_kernel(const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
                                                                     unsigned windows, unsigned log_b, unsigned log_m, xyzz *__restrict__ run_out,
                                                                     xyzz *__restrict__ streams) {
+  begin_after_previous();
   const unsigned log_g = log_b - log_m;
   const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= (windows << log_g))
@@ -547,6 +560,7 @@ __global__ void __launch_bounds__(ACC_THREADS, REDUCE_GROUPS_MIN_BLOCKS) reduce_
 __global__ void __launch_bounds__(ACC_THREADS, REDUCE_LEVEL_MIN_BLOCKS) reduce_level_kernel(const xyzz *__restrict__ t_in, xyzz *__restrict__ t_out,
                                                                    const xyzz *__restrict__ s_in, xyzz *__restrict__ s_out, unsigned windows,
                                                                    unsigned log_g, unsigned level) {
+  begin_after_previous();
   const unsigned half = (1u << log_g) >> (level + 1);
   const unsigned jobs = level + 2; // streams 0..level, then the tree
   const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -576,6 +590,7 @@ __global__ void __launch_bounds__(ACC_THREADS, REDUCE_LEVEL_MIN_BLOCKS) reduce_l
 __global__ void __launch_bounds__(ACC_THREADS) reduce_groups_group4_kernel(const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
                                                                            unsigned windows, unsigned log_b, unsigned log_m,
                                                                            xyzz *__restrict__ run_out, xyzz *__restrict__ streams) {
+  begin_after_previous();
   const unsigned log_g = log_b - log_m;
   const unsigned total = windows << log_g;
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, role = threadIdx.x & 3;
@@ -606,6 +621,7 @@ __global__ void __launch_bounds__(ACC_THREADS) reduce_groups_group4_kernel(const
 __global__ void __launch_bounds__(ACC_THREADS) reduce_level_group4_kernel(const xyzz *__restrict__ t_in, xyzz *__restrict__ t_out,
                                                                           const xyzz *__restrict__ s_in, xyzz *__restrict__ s_out, unsigned windows,
                                                                           unsigned log_g, unsigned level) {
+  begin_after_previous();
   const unsigned half = (1u << log_g) >> (level + 1);
   const unsigned jobs = level + 2; // streams 0..level, then the tree
   const unsigned total = windows * jobs * half;
@@ -644,6 +660,7 @@ __global__ void __launch_bounds__(ACC_THREADS) reduce_level_group4_kernel(const 
 __global__ void __launch_bounds__(TAIL_THREADS) reduce_tail_kernel(const xyzz *__restrict__ tree, const xyzz *__restrict__ streams,
                                                                    const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags, unsigned c,
                                                                    unsigned log_m, unsigned log_g, unsigned level, jacobian *__restrict__ results) {
+  begin_after_previous();
   const unsigned w = blockIdx.x, o = threadIdx.x;
   reduce_tail(tree, streams, w, log_g, level, [&](auto sum) {
     if (o >= c || w * c + o >= RESULT_BITS)

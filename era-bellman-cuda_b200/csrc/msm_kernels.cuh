@@ -101,6 +101,7 @@ struct plan {
   unsigned groups;      // G = B / m groups per window
   unsigned log_g;       // gamma = log2 G
   unsigned sms;         // SMs of the device the plan is for
+  bool early;           // kernels may be launched before the previous one has ended (launch_after)
   unsigned affine_levels; // affine pairing levels before the XYZZ accumulation (0: none)
   unsigned level_warps;   // warps of each level's grid
   unsigned tail_threads;  // XYZZ accumulation threads and ranges after the levels

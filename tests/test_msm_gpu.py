@@ -318,6 +318,33 @@ def test_any_window_and_length(gpu, oracle, window_bits):
     assert oracle.horner(res) == oracle.msm_checksum(k, scalars)
 
 
+@pytest.mark.parametrize("legacy", [False, True])
+def test_back_to_back(gpu, oracle, legacy):
+    """MSMs and final sums of several sizes and paths (unfused and fused digits,
+    one and two sort passes) enqueued one behind the other on one stream with
+    nothing waited for, the whole list twice over the same buffers: kernels are
+    launched before their predecessors have ended and have to wait for them.
+    On a stream of the caller's and on the legacy default stream."""
+    import bellman_cuda as bcm
+    bc, stream = gpu.bc, bcm.Handle() if legacy else gpu.stream
+    sizes = [256, 4096, 30000, 1 << 16, 5, (1 << 19) + 3]
+    scalars, k = synth.workload("uniform", max(sizes), 881 + legacy)
+    bd, _ = generated_bases(gpu, k)
+    sd = gpu.upload(scalars)
+    rd = [bc.malloc(254 * 96) for _ in sizes]
+    pd = [bc.malloc(ctypes.sizeof(bcm.AffinePoint)) for _ in sizes]
+    for _ in range(2):
+        for n, r, p in zip(sizes, rd, pd):
+            assert bc.msm_any(gpu.pool, stream, bd, sd, r, n) == 0
+            assert bc.final_sum_async(r, p, stream) == 0
+    bc.stream_synchronize(stream)
+    got = [bcm.AffinePoint.from_buffer_copy(bc.from_device(p, (20,)).tobytes()).as_tuple() for p in pd]
+    for p in [bd, sd] + rd + pd:
+        bc.free(p)
+    for n, point in zip(sizes, got):
+        assert point == oracle.msm_checksum(k[:n], scalars[:n]), n
+
+
 @pytest.mark.parametrize("window_bits", [4, 6, 7, 9, 10, 12, 14, 15, 18, 19])
 def test_reduction_tails(gpu, oracle, window_bits):
     """The widths test_any_window_and_length leaves out: the reduction's last
