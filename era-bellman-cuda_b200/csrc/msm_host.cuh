@@ -55,9 +55,6 @@ constexpr unsigned PROFILE_STAGES = 6;
 #ifndef BATCH_ACC_RANGES_PER_THREAD
 #define BATCH_ACC_RANGES_PER_THREAD 1
 #endif
-#ifndef ACC_MIN_RANGE
-#define ACC_MIN_RANGE 300 // entries a range keeps at least when ranges are multiplied
-#endif
 
 // Launches a kernel that begins with begin_after_previous().  With `early` its
 // blocks may be placed as soon as every block of the stream's previous kernel

@@ -78,6 +78,7 @@ template <unsigned THREADS, unsigned ITEMS> constexpr size_t lookback_smem_bytes
   return (size_t)THREADS * ITEMS * 8 + (size_t)(THREADS / 32) * SORT_RADIX * 4;
 }
 constexpr unsigned ACC_THREADS = 128;
+constexpr unsigned ACC_MIN_ENTRIES = 240; // per accumulation range, when a thread has several (see active_ranges)
 
 // Window w's entries start at w * window_stride(n): n rounded up to 32
 // entries, so that every window segment starts on a 128-byte line and the
