@@ -22,14 +22,15 @@
 // so 15 + 127 doublings are dependent, and about 12 additions between them.
 //
 // Levels of one or two doublings share each one between four lanes
-// (dbl_group4).  The others give a warp to each point and double it in a
-// residue number system (rns.cuh), where a product of the whole warp takes
-// less than half of one thread's: about 1,030 cycles per doubling on a B200
-// against 3,236 for dbl_group4.  The affine conversion takes one inversion
-// (inverse_group4).
-// One final sum takes 0.172 ms on a B200 (0.230 ms in one block without phi,
-// the 253 doublings one after another; 0.189 ms with the steps' code repeated),
-// of a batched instance's results (20 bits) 0.072 ms.
+// (dbl_group4).  The others give a warp to each point and double and add in a
+// residue number system (rns.cuh), where a product of the whole warp takes less
+// than half of one thread's: about 1,030 cycles per doubling on a B200 against
+// 3,236 for dbl_group4.  The affine conversion takes one inversion
+// (inverse_group4).  One final sum takes 0.157 ms on a B200, of a batched
+// instance's results (20 bits) 0.068 ms.  Measured on the way there: 0.230 ms in
+// one block without phi, the 253 doublings one after another; 0.189 ms with the
+// steps' code repeated; 0.169 ms with four-lane additions (and a conversion out
+// of the residues and back) at every level.
 #include "bellman-cuda-b200.h"
 #include "msm_device.cuh"
 #include "msm_group4.cuh"
@@ -73,11 +74,15 @@ __device__ __forceinline__ fe endomorphism_beta() {
 
 __device__ const rns::tables rns_tables = rns::TABLES;
 
-// Doublings of one point by a whole warp.  All lanes hold their residues of X
-// and Y of a Jacobian point, the lanes of groups 1 and 2 those of Z
-// (x = X / Z^2, y = Y / Z^3).
+// Doublings and additions of points by a whole warp.  All lanes hold their
+// residues of X and Y of a Jacobian point, the lanes of groups 1 and 2 those of
+// Z (x = X / Z^2, y = Y / Z^3; infinity: Z = 0 mod p).
 struct rns_point {
   rns::residues x, y, z;
+};
+// the same between steps, one entry per residue index
+struct rns_stored {
+  rns::residues x[rns::RESIDUES], y[rns::RESIDUES], z[rns::RESIDUES];
 };
 
 struct rns_warp {
@@ -149,6 +154,45 @@ struct rns_warp {
     return {from_group(x, 0), from_group(y, 0), rns::scaled(r3, 2)};
   }
 
+  // p + q, six products deep (add-2007-bl without its doublings):
+  //   Z1^2 | Z2^2 | Z1 Z2;  U1 = X1 Z2^2 | U2 = X2 Z1^2 | Z2^3;
+  //   S1 = Y1 Z2^3 | Z1^3 | H^2, H = U2 - U1;  S2 = Y2 Z1^3 | H^3 | V = U1 H^2;
+  //   R^2 | S1 H^3 | Z3 = Z1 Z2 H, R = S2 - S1;
+  //   R (V - X3) with X3 = R^2 - H^3 - 2 V;  Y3 = that - S1 H^3.
+  // false when Z3 is zero (an infinite operand, equal or opposite points): the
+  // formula does not hold then.  Sums stay below those of doubled().
+  __device__ __forceinline__ bool added(const rns_point &p, const rns_point &q, rns_point &sum) const {
+    const rns::residues z1 = from_group(p.z, 1), z2 = from_group(q.z, 1);
+    const rns::residues r1 = product(pick(z1, z2, z1), pick(z1, z2, z2));
+    const rns::residues zz1 = from_group(r1, 0), zz2 = from_group(r1, 1);
+    const rns::residues r2 = product(pick(p.x, q.x, z2), pick(zz2, zz1, zz2));
+    const rns::residues U1 = from_group(r2, 0), H = from_group(r2, 1) - U1;
+    const rns::residues r3 = product(pick(p.y, z1, H), pick(from_group(r2, 2), zz1, H));
+    const rns::residues HH = from_group(r3, 2), S1 = from_group(r3, 0);
+    const rns::residues r4 = product(pick(q.y, H, U1), pick(from_group(r3, 1), HH, HH));
+    const rns::residues R = from_group(r4, 0) - S1, HHH = from_group(r4, 1), V = from_group(r4, 2);
+    const rns::residues r5 = product(pick(R, S1, r1), pick(R, HHH, H));
+    const uint32_t zero = __reduce_and_sync(0xffffffffu, group == 2 ? rns::multiples_of_p(t, r5) : 0xffffffffu);
+    const rns::residues x = from_group(r5, 0) - HHH - rns::scaled(V, 2);
+    const rns::residues y = product(R, V - x) - from_group(r5, 1);
+    sum = {x, y, from_group(r5, 2)};
+    return (zero & 0x007f007fu) == 0;
+  }
+
+  __device__ __forceinline__ void put(rns_stored &to, const rns_point &p) const {
+    const rns::residues z = from_group(p.z, 1);
+    if ((threadIdx.x & 31) < rns::RESIDUES) {
+      const unsigned i = threadIdx.x & 31;
+      to.x[i] = p.x;
+      to.y[i] = p.y;
+      to.z[i] = z;
+    }
+  }
+  __device__ __forceinline__ rns_point get(const rns_stored &from) const {
+    const unsigned i = (threadIdx.x & 31) - base;
+    return {from.x[i], from.y[i], from.z[i]};
+  }
+
   // X, Y, Z as Montgomery-form field elements in (0, 2p), the same in every
   // lane; columns: 24 words of shared memory of this warp
   __device__ __forceinline__ jacobian store(const rns_point &p, int64_t (*columns)[8]) const {
@@ -175,6 +219,8 @@ struct final_shared {
   xyzz part[FINAL_PARTS];
   xyzz group[GROUPS];            // every block's two group sums
   xyzz choice[SPLIT_GROUPS][3];  // of a split group, signed: V, phi(V), their sum
+  rns_stored stored[FINAL_PARTS]; // parts between two steps of a warp per point
+  bool empty[FINAL_PARTS];        // infinite ones among them
   int64_t columns[FINAL_WARPS][rns::GROUPS][8];
 };
 
@@ -253,8 +299,16 @@ __global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THR
       sum_digits(sh, rank);
     } else if (step == 8) {
       cluster.sync();
-      if (rank == 0 && t >= 8 && t < 8 * FINAL_BLOCKS) // block k's sum, of bits from 16 k on, into part 2 k
-        copy_remote(cluster, &sh.part[2 * (t >> 3)], &sh.part[0], t >> 3, t & 7);
+      if (rank == 0 && t >= 32) { // block k's sum, of bits from 16 k on, into part 2 k
+        constexpr unsigned WORDS = sizeof(rns_stored) / 8;
+        for (unsigned q = t - 32; q < (FINAL_BLOCKS - 1) * WORDS; q += FINAL_THREADS - 32) {
+          const unsigned k = 1 + q / WORDS;
+          reinterpret_cast<uint2 *>(&sh.stored[2 * k])[q % WORDS] =
+              reinterpret_cast<const uint2 *>(cluster.map_shared_rank(&sh.stored[0], k))[q % WORDS];
+        }
+        if (t - 32 < FINAL_BLOCKS - 1)
+          sh.empty[2 * (t - 31)] = *cluster.map_shared_rank(&sh.empty[0], t - 31);
+      }
       cluster.sync(); // the other blocks stay until their sums are read
       if (rank != 0)
         return;
@@ -263,9 +317,9 @@ __global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THR
     const unsigned n = step < 4 ? 1u << level : step < 8 ? 1u << (level - 1) : 4u << level;
     const unsigned pairs = FINAL_PARTS >> level, half = (1u << level) >> 1;
     const bool by_lanes = n < FINAL_RNS_DOUBLINGS; // four lanes per pair, or a warp
-    if ((by_lanes ? (t & ~31u) >> 2 : t >> 5) < pairs) { // the warp has a pair; groups of lanes without one redo the first
-      const bool active = !by_lanes || t >> 2 < pairs;
-      const unsigned pair = by_lanes ? (active ? t >> 2 : 0) : t >> 5, target = pair << level;
+    if (by_lanes && (t & ~31u) >> 2 < pairs) { // the warp has a pair; groups of lanes without one redo the first
+      const bool active = t >> 2 < pairs;
+      const unsigned pair = active ? t >> 2 : 0, target = pair << level;
       xyzz q, o;
       if (step == 0) {
         const unsigned r = 2 * (rank * FINAL_PARTS + pair);
@@ -285,22 +339,64 @@ __global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THR
       }
       // an infinite partner adds nothing (the batched path's results are infinity above bit c - 1)
       if (!__all_sync(0xffffffffu, curve::is_inf(o))) {
-        if (by_lanes) {
 #pragma unroll 1
-          for (unsigned k = 0; k < n; k++)
-            o = dbl_group4(o);
-        } else {
-          rns_point d = w.load(sh.part[target + half]);
-#pragma unroll 1
-          for (unsigned k = 0; k < n; k++)
-            d = w.doubled(d);
-          o = curve::from_jacobian(w.store(d, sh.columns[t >> 5]));
-        }
+        for (unsigned k = 0; k < n; k++)
+          o = dbl_group4(o);
         q = add_group4(q, o);
       }
       __syncwarp();
-      if (active && (by_lanes ? role == 0 : (t & 31) == 0))
+      if (active && role == 0)
         sh.part[target] = q;
+    }
+    if (!by_lanes && t >> 5 < pairs) {
+      // steps 2 and 6 start from part[], 3 and 10 end there; between, the
+      // points stay residues
+      const bool enters = step == 2 || step == 6, leaves = step == 3 || step == 10;
+      const unsigned target = (t >> 5) << level, partner = target + half;
+      bool empty = enters ? curve::is_inf(sh.part[target]) : sh.empty[target];
+      const bool adds = !(enters ? curve::is_inf(sh.part[partner]) : sh.empty[partner]);
+      rns_point q{}, o{};
+#pragma unroll 1
+      for (unsigned k = empty; k <= adds; k++) { // 0: the target, 1: its partner
+        const rns_point p = enters ? w.load(sh.part[k ? partner : target]) : w.get(sh.stored[k ? partner : target]);
+        if (k)
+          o = p;
+        else
+          q = p;
+      }
+      if (adds) {
+#pragma unroll 1
+        for (unsigned k = 0; k < n; k++)
+          o = w.doubled(o);
+        rns_point sum;
+        if (empty) {
+          q = o;
+          empty = false;
+        } else if (w.added(q, o, sum)) {
+          q = sum;
+        } else { // equal or opposite points
+          const jacobian a = w.store(q, sh.columns[t >> 5]), b = w.store(o, sh.columns[t >> 5]);
+          const xyzz s = add_group4(curve::from_jacobian(a), curve::from_jacobian(b));
+          __syncwarp();
+          if ((t & 31) == 0)
+            sh.part[target] = s;
+          __syncwarp();
+          q = w.load(sh.part[target]);
+          empty = curve::is_inf(s);
+        }
+      }
+      __syncwarp();
+      if (leaves) {
+        xyzz p = curve::infinity();
+        if (!empty)
+          p = curve::from_jacobian(w.store(q, sh.columns[t >> 5]));
+        if ((t & 31) == 0)
+          sh.part[target] = p;
+      } else {
+        w.put(sh.stored[target], q);
+        if ((t & 31) == 0)
+          sh.empty[target] = empty;
+      }
     }
     __syncthreads();
   }

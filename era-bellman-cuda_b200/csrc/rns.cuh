@@ -49,6 +49,7 @@ struct lane_table {
   int32_t value;                  // (B / b_i) 2^64 mod b_i
   int32_t whole;                  // -B 2^64 mod a_i
   int32_t p_b;                    // (B / b_i)^-1 p 2^32 mod b_i
+  uint32_t p_a;                   // p as a stored residue modulo a_i, in [0, a_i)
   int32_t to_b[RESIDUES];         // (B / b_i)^-1 (A / a_k) p / A 2^32 mod b_i
   int32_t to_a[RESIDUES];         // (B / b_k) 2^64 mod a_i
   uint32_t word_a[8], word_b[8];  // 2^(32 k + 64) mod a_i, b_i, in [0, modulus)
@@ -176,6 +177,7 @@ struct table_builder {
       l.whole = centred(ma - mulmod(product(b, RESIDUES, ma), two_to(64, ma), ma), ma);
       const uint32_t zeta_p = mulmod(mulmod(words_mod(p, mb), zeta, mb), two_to(32, mb), mb);
       l.p_b = centred(zeta_p, mb);
+      l.p_a = mulmod(words_mod(p, ma), two_to(32, ma), ma);
       for (unsigned k = 0; k < RESIDUES; k++) {
         l.to_b[k] = centred(mulmod(mulmod(product(a, k, mb), inv_a, mb), zeta_p, mb), mb);
         l.to_a[k] = centred(mulmod(product(b, k, ma), two_to(64, ma), ma), ma);
@@ -265,6 +267,20 @@ template <class EXTEND> BN_HD residues product(const lane_table &t, const residu
   });
   back += (int64_t)((all + (1 << 26)) >> 27) * t.whole;
   return {word_redc(back, t.mod_a, t.ninv_a), word_redc((int64_t)zeta * t.value, t.mod_b, t.ninv_b)};
+}
+
+// A product's output is a multiple k p, |k| <= 6 (zero in the field), iff
+// every lane of the group finds its residue equal for the same k: bit k of the
+// result says so for this lane's residue and k, bit 16 + k for -k.
+BN_HD uint32_t multiples_of_p(const lane_table &t, const residues &r) {
+  const uint32_t m = (uint32_t)t.mod_a, c = (uint32_t)(r.a < 0 ? r.a + t.mod_a : r.a);
+  uint32_t found = 0, kp = 0;
+  for (unsigned k = 0; k <= 6; k++) {
+    found |= (uint32_t)(c == kp) << k | (uint32_t)(c == (kp ? m - kp : 0)) << (16 + k);
+    kp += t.p_a;
+    kp = kp >= m ? kp - m : kp;
+  }
+  return found;
 }
 
 // Word column `lane` (lane < 8) of p + (x y + q p) / A, q taken nearest to

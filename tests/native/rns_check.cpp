@@ -72,6 +72,14 @@ void rns_product_words(const int32_t *x, const int32_t *y, uint32_t *out) {
   }
 }
 
+// the warp's test for a multiple of p: the lanes' words and-ed
+uint32_t rns_multiples(const int32_t *x) {
+  uint32_t all = 0xffffffffu;
+  for (int i = 0; i < N; i++)
+    all &= rns::multiples_of_p(rns::TABLES.lane[i], {x[i], x[N + i]});
+  return all;
+}
+
 void rns_constants(int32_t *enter, int32_t *leave) {
   for (int i = 0; i < N; i++) {
     enter[i] = rns::TABLES.lane[i].enter_a;

@@ -208,3 +208,20 @@ def test_doubling_chains(gpu, oracle, bits):
     zs = [int.from_bytes(rng.bytes(32), "little") % P or 1 for _ in range(254)]
     res = results_of(pts, zs)
     assert final_sum(gpu, res) == oracle.horner(res)
+
+
+@pytest.mark.parametrize("bit", [2, 4, 8, 16, 32, 64])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_equal_and_opposite_partners(gpu, oracle, bit, sign):
+    """2^bit G against +-(G at that bit): the two operands of one tree level's
+    addition are equal or opposite (bits 2: four lanes per point; the others a
+    warp per point, in the groups up to 8 and across them from 16), alone and
+    with a result above it."""
+    G = H.load_g_bases()[0]
+    inf, *big = oracle.affine_mul(G[0], G[1], 1 << bit)
+    assert not inf
+    pts = {0: tuple(big), bit: G if sign > 0 else neg(G)}
+    zs = [3 + i for i in range(254)]
+    for extra in ({}, {100: G}, {253: G}):
+        res = results_of({**pts, **extra}, zs)
+        assert final_sum(gpu, res) == oracle.horner(res), (bit, sign, extra)

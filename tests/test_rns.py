@@ -151,3 +151,52 @@ def test_doubling_chain(rns):
     inv = pow(rns.A, -1, P)
     assert [rns.value(v) * inv % P for v in (X, Y, Z)] == [x, y, z]
     assert most_word < 13 * 1.25 * 2 ** 26 and most_value < 85 * P
+
+
+def test_multiples_of_p(rns):
+    """A product's output is recognised as k p, |k| <= 6, and only then."""
+    rng = random.Random(9)
+    one = rns.enter(1)
+    is_multiple = lambda x: (rns.lib.rns_multiples(np.ascontiguousarray(x, np.int32).ctypes.data_as(ctypes.c_void_p)) & 0x007F007F) != 0
+    for trial in range(200):
+        x = rng.randrange(P)
+        zero = rns.product(rns.enter(P) if trial % 2 else rns.enter(0), rns.enter(x))  # (p or 0) x: some multiple of p
+        assert rns.value(zero) % P == 0 and is_multiple(zero)
+        other = rns.product(rns.enter(x), one)
+        assert is_multiple(other) == (x == 0)
+    stored_p = rns.enter(P)
+    for k in range(-6, 7):  # every multiple, with words reduced as a product's are
+        words = []
+        for part, mods in ((stored_p[:rns.n], rns.a), (stored_p[rns.n:], rns.b)):
+            words += [((int(w) * k + m // 2) % m) - m // 2 for w, m in zip(part, mods)]
+        assert is_multiple(np.array(words))
+        near = list(words)
+        near[3] += 1 if near[3] <= 0 else -1
+        assert not is_multiple(np.array(near))
+
+
+def test_additions(rns):
+    """The final sum's addition on doubled and added operands, 60 times over."""
+    rng = random.Random(10)
+    inv = pow(rns.A, -1, P)
+    p, q = ([rng.randrange(1, P) for _ in range(3)] for _ in range(2))
+    Pt, Qt = ([rns.enter(v * rns.A % P) for v in pt] for pt in (p, q))
+    for step in range(60):
+        (x1, y1, z1), (x2, y2, z2) = Pt, Qt
+        zz1, zz2, z12 = rns.product(z1, z1), rns.product(z2, z2), rns.product(z1, z2)
+        U1, U2, z2c = rns.product(x1, zz2), rns.product(x2, zz1), rns.product(z2, zz2)
+        H = U2 - U1
+        S1, z1c, HH = rns.product(y1, z2c), rns.product(z1, zz1), rns.product(H, H)
+        S2, HHH, V = rns.product(y2, z1c), rns.product(H, HH), rns.product(U1, HH)
+        R = S2 - S1
+        RR, T, Z = rns.product(R, R), rns.product(S1, HHH), rns.product(z12, H)
+        X = RR - HHH - 2 * V
+        Y = rns.product(R, V - X) - T
+        (a, b, c), (d, e, f) = p, q
+        h, r = (d * c * c - a * f * f) % P, (e * c ** 3 - b * f ** 3) % P
+        v = a * f * f * h * h % P
+        x = (r * r - h ** 3 - 2 * v) % P
+        want = [x, (r * (v - x) - b * f ** 3 * h ** 3) % P, c * f * h % P]
+        assert [rns.value(w) * inv % P for w in (X, Y, Z)] == want
+        assert max(int(np.abs(w.astype(np.int64)).max()) for w in (H, R, X, V - X, Y)) < 13 * 1.25 * 2 ** 26
+        p, q, Pt, Qt = q, want, Qt, [X, Y, Z]
