@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(SORT_THREADS) batch_digits_histogram_kernel(co
                                                                               uint32_t *__restrict__ counts, uint32_t *__restrict__ zeros,
                                                                               unsigned instances, unsigned later_passes,
                                                                               uint32_t *__restrict__ later_totals) {
+  begin_after_previous();
   // [windows][SORT_RADIX] first-pass counters, [later_passes][SORT_RADIX], then the zero-digit count
   extern __shared__ uint32_t s_hist[];
   const unsigned k = ptile_seg[blockIdx.x];
@@ -198,6 +199,7 @@ static size_t batch_digit_smem(unsigned c, unsigned later_passes) {
 // one warp per (segment, digit) row
 __global__ void __launch_bounds__(256) batch_sort_scan_kernel(uint32_t *counts, const batch_instance *__restrict__ inst, unsigned rows,
                                                               uint32_t *__restrict__ totals) {
+  begin_after_previous();
   const unsigned row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= rows)
     return;
@@ -210,6 +212,7 @@ __global__ void __launch_bounds__(SORT_THREADS, SORT_SCATTER_MIN_BLOCKS) batch_s
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
     const batch_instance *__restrict__ inst, const unsigned *__restrict__ tile_seg, const uint32_t *__restrict__ counts,
     const uint32_t *__restrict__ totals, const uint32_t *__restrict__ zeros) {
+  begin_after_previous();
   const unsigned t = blockIdx.x;
   const unsigned k = tile_seg[t];
   const batch_instance d = inst[k];
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(SORT_THREADS, SORT_SCATTER_MIN_BLOCKS) batch_l
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
     const batch_instance *__restrict__ inst, const unsigned *__restrict__ tile_seg, const unsigned *__restrict__ tile_order, unsigned shift,
     uint32_t *words, const uint32_t *__restrict__ totals, const uint32_t *__restrict__ zeros, unsigned *tile_ctr, unsigned *error) {
+  begin_after_previous();
   __shared__ unsigned s_ticket;
   if (threadIdx.x == 0)
     s_ticket = atomicAdd(tile_ctr, 1u);
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(ACC_THREADS, ACC_MIN_BLOCKS) batch_accumulate_
     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, const batch_instance *__restrict__ inst, unsigned instances,
     const uint32_t *__restrict__ zeros, unsigned ranges, unsigned *__restrict__ work, xyzz *__restrict__ buckets, uint8_t *__restrict__ flags,
     uint32_t *__restrict__ head_bucket, xyzz *__restrict__ head_point) {
+  begin_after_previous();
   __shared__ unsigned long long s_first[MAX_BATCH], s_end[MAX_BATCH], s_prefix[MAX_BATCH + 1];
   __shared__ uint32_t s_bucket[MAX_BATCH], s_mask[MAX_BATCH];
   __shared__ const affine *s_table[MAX_BATCH];
@@ -303,6 +308,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) batch_reduce_tail_kernel(const x
                                                                          const xyzz *__restrict__ buckets, const uint8_t *__restrict__ flags,
                                                                          const unsigned *__restrict__ members, unsigned c, unsigned log_m,
                                                                          unsigned log_g, unsigned level, const batch_io *__restrict__ io) {
+  begin_after_previous();
   const unsigned w = blockIdx.x, i = threadIdx.x;
   reduce_tail(tree, streams, w, log_g, level, [&](auto sum) {
     if (i >= RESULT_BITS)
@@ -632,7 +638,7 @@ std::vector<uint8_t> descriptor_image(const batch_plan &b) {
 // stream and one event per reduction group, plus one event), the per-width
 // reductions run concurrently; otherwise one after another on s.
 cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s, const cudaStream_t *forks, const cudaEvent_t *fork_events,
-                                 unsigned *launches) {
+                          bool early, unsigned *launches) {
   auto at = [&](size_t off) { return scratch + off; };
   unsigned launched = 0;
   uint32_t *keys[2] = {reinterpret_cast<uint32_t *>(at(b.keys[0])), reinterpret_cast<uint32_t *>(at(b.keys[1]))};
@@ -652,16 +658,14 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
   const unsigned later = b.sort_passes - 1;
   uint32_t *later_totals = reinterpret_cast<uint32_t *>(at(b.later_totals));
   // digits, with the first pass's counts per sort tile and the later passes' digit totals
-  batch_digits_histogram_kernel<<<b.total_point_tiles, SORT_THREADS, b.digit_smem, s>>>(
-      inst, reinterpret_cast<const unsigned *>(at(b.ptile_seg_dev)), io, keys[0], vals[0], counts, zeros, b.instances, later, later_totals);
-  CHECK(cudaGetLastError());
+  CHECK(launch_after(early, batch_digits_histogram_kernel, b.total_point_tiles, SORT_THREADS, b.digit_smem, s, inst,
+                     reinterpret_cast<const unsigned *>(at(b.ptile_seg_dev)), io, keys[0], vals[0], counts, zeros, b.instances, later, later_totals));
   launched++;
   // the first pass: tile offsets and digit totals by one scan, then the scatter (drops zero digits)
   const unsigned rows = b.instances * SORT_RADIX;
-  batch_sort_scan_kernel<<<(rows * 32 + 255) / 256, 256, 0, s>>>(counts, inst, rows, totals);
-  CHECK(cudaGetLastError());
-  batch_sort_scatter_first_kernel<<<b.total_tiles, SORT_THREADS, 0, s>>>(keys[0], vals[0], keys[1], vals[1], inst, tile_seg, counts, totals, zeros);
-  CHECK(cudaGetLastError());
+  CHECK(launch_after(early, batch_sort_scan_kernel, (rows * 32 + 255) / 256, 256, 0, s, counts, inst, rows, totals));
+  CHECK(launch_after(early, batch_sort_scatter_first_kernel, b.total_tiles, SORT_THREADS, 0, s, keys[0], vals[0], keys[1], vals[1], inst, tile_seg,
+                     counts, totals, zeros));
   launched += 2;
   int cur = 1;
   // later passes: one look-back kernel each, on words cleared before it
@@ -671,25 +675,24 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
   for (unsigned pass = 1; pass < b.sort_passes; pass++) {
     uint32_t *words = pass == 1 ? counts : reinterpret_cast<uint32_t *>(at(b.words2));
     CHECK(cudaMemsetAsync(words, 0, word_bytes, s));
-    batch_lookback_kernel<<<b.total_tiles, SORT_THREADS, lookback_smem_bytes<SORT_THREADS, SORT_ITEMS>(), s>>>(
-        keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], inst, tile_seg, tile_order, pass * SORT_RADIX_BITS, words,
-        later_totals + (size_t)(pass - 1) * b.instances * SORT_RADIX, zeros, sort_ctrs + pass - 1, sort_error);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(early, batch_lookback_kernel, b.total_tiles, SORT_THREADS, lookback_smem_bytes<SORT_THREADS, SORT_ITEMS>(), s, keys[cur],
+                       vals[cur], keys[cur ^ 1], vals[cur ^ 1], inst, tile_seg, tile_order, pass * SORT_RADIX_BITS, words,
+                       later_totals + (size_t)(pass - 1) * b.instances * SORT_RADIX, zeros, sort_ctrs + pass - 1, sort_error));
     launched++;
     cur ^= 1;
   }
   unsigned *work = reinterpret_cast<unsigned *>(at(b.work));
   CHECK(cudaMemsetAsync(work, 0, sizeof(unsigned), s));
-  batch_accumulate_kernel<<<(b.acc_threads + ACC_THREADS - 1) / ACC_THREADS, ACC_THREADS, 0, s>>>(
-      keys[cur], vals[cur], inst, b.instances, zeros, b.acc_ranges, work, buckets, flags, hb[0], hp[0]);
-  CHECK(cudaGetLastError());
+  CHECK(launch_after(early, batch_accumulate_kernel, (b.acc_threads + ACC_THREADS - 1) / ACC_THREADS, ACC_THREADS, 0, s, keys[cur], vals[cur], inst,
+                     b.instances, zeros, b.acc_ranges, work, buckets, flags, hb[0], hp[0]));
   launched++;
-  CHECK(enqueue_merge_heads(hb, hp, b.acc_ranges, buckets, b.sms, false, s, launched));
+  CHECK(enqueue_merge_heads(hb, hp, b.acc_ranges, buckets, b.sms, early, s, launched));
   if (forks)
     CHECK(cudaEventRecord(fork_events[0], s));
   for (size_t g = 0; g < b.groups.size(); g++) {
     const batch_group &grp = b.groups[g];
-    const plan &p = grp.p;
+    plan p = grp.p;
+    p.early = early;
     cudaStream_t fs = forks ? forks[g] : s;
     if (forks)
       CHECK(cudaStreamWaitEvent(fs, fork_events[0], 0));
@@ -699,10 +702,8 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
     xyzz *const streams[2] = {reinterpret_cast<xyzz *>(at(grp.streams[0])), reinterpret_cast<xyzz *>(at(grp.streams[1]))};
     CHECK(enqueue_window_sums(p, gb, gf, tree, streams, fs, launched));
     const unsigned level = tail_level(p.log_g);
-    batch_reduce_tail_kernel<<<p.windows, TAIL_THREADS, tail_smem(p.log_g), fs>>>(tree[level & 1], streams[level & 1], gb, gf,
-                                                                                  reinterpret_cast<const unsigned *>(at(grp.members_dev)), p.c,
-                                                                                  p.log_m, p.log_g, level, io);
-    CHECK(cudaGetLastError());
+    CHECK(launch_after(early, batch_reduce_tail_kernel, p.windows, TAIL_THREADS, tail_smem(p.log_g), fs, tree[level & 1], streams[level & 1], gb, gf,
+                       reinterpret_cast<const unsigned *>(at(grp.members_dev)), p.c, p.log_m, p.log_g, level, io));
     launched++;
     if (forks) {
       CHECK(cudaEventRecord(fork_events[g + 1], fs));
@@ -787,7 +788,7 @@ cudaError_t batch_create(batch_impl **out, const base_table_impl *table, const u
   for (auto &e : bi.fork_events)
     CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   CHECK(cudaStreamBeginCapture(bi.capture, cudaStreamCaptureModeThreadLocal));
-  const cudaError_t enq = enqueue_batch(b, bi.scratch, bi.capture, bi.forks.data(), bi.fork_events.data(), &bi.launches);
+  const cudaError_t enq = enqueue_batch(b, bi.scratch, bi.capture, bi.forks.data(), bi.fork_events.data(), false, &bi.launches);
   cudaGraph_t graph = nullptr;
   const cudaError_t end = cudaStreamEndCapture(bi.capture, &graph);
   bi.graph = graph;

@@ -78,9 +78,10 @@ cudaError_t make_batch_plan(batch_plan &b, const base_table_impl *table, const u
 // the constant descriptors as they lie in scratch from b.descriptors on
 std::vector<uint8_t> descriptor_image(const batch_plan &b);
 // the chain of plan b over `scratch`; forks (optional): one stream per
-// reduction group and groups + 1 events, for concurrent reductions
+// reduction group and groups + 1 events, for concurrent reductions; early: see
+// launch_after (not for a stream that is being captured)
 cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s, const cudaStream_t *forks, const cudaEvent_t *fork_events,
-                          unsigned *launches);
+                          bool early, unsigned *launches);
 // writes the instances' scalar and result pointers into the io table
 cudaError_t enqueue_io(batch_io *io, unsigned instances, const void *const *scalars, void *const *results, cudaStream_t stream);
 cudaError_t batch_set_up();

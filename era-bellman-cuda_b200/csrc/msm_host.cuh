@@ -64,8 +64,8 @@ constexpr unsigned PROFILE_STAGES = 6;
 // 0.532, 2^18 1.110 -> 1.057, 2^22 10.802 -> 10.748.  Kernels that let the next
 // one start at their own start (griddepcontrol.launch_dependents) were slower,
 // 2^12 0.198 and 2^18 1.185 ms: the next kernel's blocks then pile up on the
-// SMs that are free at that moment.  A captured batch is launched plainly: its
-// graph took the same time either way (2.702 against 2.706 ms).
+// SMs that are free at that moment.  A batch that is captured records plain
+// kernels: its graph took the same time either way (2.702 against 2.706 ms).
 template <class... P, class... A>
 cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchAttribute attribute{};
