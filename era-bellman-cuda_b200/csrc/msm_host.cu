@@ -302,7 +302,8 @@ static layout make_layout(const plan &p, bool copy_scalars, bool copy_bases, boo
   // the first pass's digit counts per (window, digit, tile); then one region
   // cleared per chunk: digit totals per (pass, window, digit), zero digits
   // per window, a tile counter per pass, the look-back error word, the
-  // accumulation's work counter, and the
+  // accumulation's work counter (from the zero counts up to here cleared by
+  // digits_kernel where that runs), and the
   // look-back words of the passes after the first, per (window, look-back
   // tile, digit)
   const size_t lookback_words = (size_t)p.windows * p.lookback_tiles * SORT_RADIX;
@@ -322,9 +323,10 @@ static layout make_layout(const plan &p, bool copy_scalars, bool copy_bases, boo
     l.chunk_flags = take(slots);
   }
   const size_t heads = std::max(p.acc_ranges, p.tail_ranges);
-  for (int i = 0; i < 2; i++) {
-    l.hb[i] = take(heads * 4);
-    l.hp[i] = take(heads * sizeof(xyzz));
+  for (int i = 0; i < 2; i++) { // the second pair holds a merge level's output
+    const size_t count = i ? (heads + MERGE_HEADS_PER_WARP_GROUP4 - 1) / MERGE_HEADS_PER_WARP_GROUP4 : heads;
+    l.hb[i] = take(count * 4);
+    l.hp[i] = take(count * sizeof(xyzz));
   }
   if (p.affine_levels) {
     const unsigned long long entries = (unsigned long long)p.windows * p.n, slots = (unsigned long long)p.windows << p.log_b;
@@ -416,8 +418,7 @@ struct stage_marks {
 };
 
 // Stages 1-5 for the points of one plan: digits, sort, zero counts,
-// accumulation and head merge into (buckets, flags).  Flags must be zero for
-// buckets that hold nothing yet.
+// accumulation and head merge into (buckets, flags), flags cleared first.
 static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const affine *bases, xyzz *buckets, uint8_t *flags, uint8_t *scratch,
                                         const layout &l, cudaStream_t stream, stage_marks &m) {
   uint32_t *keys[2] = {reinterpret_cast<uint32_t *>(scratch + l.keys[0]), reinterpret_cast<uint32_t *>(scratch + l.keys[1])};
@@ -431,10 +432,12 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
 
   unsigned *sort_ctrs = reinterpret_cast<unsigned *>(scratch + l.sort_ctrs);
   unsigned *sort_error = reinterpret_cast<unsigned *>(scratch + l.sort_error);
-  CHECK(cudaMemsetAsync(totals, 0, l.sort_clear_bytes, stream));
+  const size_t slots = (size_t)p.windows << p.log_b;
   int cur = 0;
   if (p.windows <= MAX_FUSED_HISTOGRAM_WINDOWS && p.tiles >= FUSED_DIGITS_MIN_TILES) {
     // 1. digits, with every pass's digit counts per tile
+    CHECK(cudaMemsetAsync(flags, 0, slots, stream));
+    CHECK(cudaMemsetAsync(totals, 0, l.sort_clear_bytes, stream));
     CHECK(launch_after(p.early, digits_histogram_kernel, p.tiles, SORT_THREADS, digit_histogram_smem(p.windows, p.sort_passes), stream, scalars, n,
                        p.c, p.windows, p.sort_passes, p.tiles, keys[0], vals[0], counts, totals, zeros));
     m.launched++;
@@ -460,7 +463,9 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
     }
   } else {
     // 1. digits (c <= 5: more windows than the digit kernel can count)
-    CHECK(launch_after(p.early, digits_kernel, (n + 255) / 256, 256, 0, stream, scalars, n, p.c, p.windows, keys[0], vals[0]));
+    const cleared_words counters = {zeros, (unsigned)((l.lookback_words - l.zeros) / 4)}; // zero counts .. work counter
+    const cleared_words flag_words = {reinterpret_cast<uint32_t *>(flags), (unsigned)((slots + 3) / 4)};
+    CHECK(launch_after(p.early, digits_kernel, (n + 255) / 256, 256, 0, stream, scalars, n, p.c, p.windows, keys[0], vals[0], counters, flag_words));
     m.launched++;
     CHECK(m.mark(stream));
     // 2. sort, 8 bits per pass: histogram, scan and scatter kernels
@@ -630,7 +635,6 @@ cudaError_t enqueue_pipeline(const plan &p, const fe *scalars, const affine *bas
   m.events = stage_events;
   xyzz *buckets = reinterpret_cast<xyzz *>(scratch + l.buckets);
   uint8_t *flags = scratch + l.flags;
-  CHECK(cudaMemsetAsync(flags, 0, (size_t)p.windows << p.log_b, stream));
   CHECK(m.mark(stream));
   CHECK(enqueue_accumulation(p, scalars, bases, buckets, flags, scratch, l, stream, m));
   CHECK(enqueue_reduction(p, buckets, flags, results, scratch, l, stream, m));
@@ -755,7 +759,6 @@ static cudaError_t enqueue_chunked(const execution &e, const chunking &ch, const
   uint8_t *chunk_flags = scratch + l.chunk_flags;
   const size_t slots = (size_t)full.windows << full.log_b;
   stage_marks m;
-  CHECK(cudaMemsetAsync(flags, 0, slots, stream));
   // copy j + 1 is enqueued before chunk j's kernels, so that the host thread
   // (which stages pageable copies itself) never holds back enqueued work
   if (copying)
@@ -773,7 +776,6 @@ static cudaError_t enqueue_chunked(const execution &e, const chunking &ch, const
     if (j == 0) {
       CHECK(enqueue_accumulation(p, src_scalars, src_bases, buckets, flags, scratch, l, stream, m));
     } else {
-      CHECK(cudaMemsetAsync(chunk_flags, 0, slots, stream));
       CHECK(enqueue_accumulation(p, src_scalars, src_bases, chunk_buckets, chunk_flags, scratch, l, stream, m));
       CHECK(launch_after(full.early, merge_chunk_buckets_kernel, (unsigned)((slots + ACC_THREADS - 1) / ACC_THREADS), ACC_THREADS, 0, stream, buckets,
                          flags, chunk_buckets, chunk_flags, (unsigned)slots));
@@ -1008,9 +1010,12 @@ cudaError_t execute_no_alloc(cudaStream_t stream, const void *bases, const void 
   plan p = make_plan(count, 0, get_device_info(device).sms);
   p.early = early_launches(stream);
   set_affine_levels(p, 0);   // the fixed scratch holds no level lists
-  set_reduction_groups(p, 3); // and the reduction's smallest tree (G = B / 8)
-  const layout l = make_layout(p, false, false, false);
-  if (l.total > MSM_B200_NO_ALLOC_SCRATCH_BYTES) // only on GPUs far larger than a B200 (heads grow with the SM count)
+  layout l = make_layout(p, false, false, false);
+  if (l.total > MSM_B200_NO_ALLOC_SCRATCH_BYTES) { // on GPUs larger than a B200 (heads grow with the SM count): the smallest tree, G = B / 8
+    set_reduction_groups(p, 3);
+    l = make_layout(p, false, false, false);
+  }
+  if (l.total > MSM_B200_NO_ALLOC_SCRATCH_BYTES)
     return cudaErrorInvalidValue;
   uint8_t *scratch = nullptr;
   CHECK(no_alloc_scratch_address(&scratch));
