@@ -105,7 +105,7 @@ struct server_impl {
   double now_us() const { return std::chrono::duration<double, std::micro>(clock_type::now() - t0).count(); }
   ~server_impl();
   void run();
-  bool admit_one(slot &s); // called with lock held
+  bool admit_one(slot &s, std::unique_lock<std::mutex> &held); // called with the lock held; released while the group is enqueued
 };
 
 static bool is_host(const void *ptr, cudaError_t &err) {
@@ -133,7 +133,7 @@ static size_t staged_bytes(const std::vector<request *> &members) {
   return bytes;
 }
 
-bool server_impl::admit_one(slot &s) {
+bool server_impl::admit_one(slot &s, std::unique_lock<std::mutex> &held) {
   if (pending.empty())
     return false;
   // The group is the longest prefix of the queue whose footprint fits.  Mostly
@@ -206,7 +206,11 @@ bool server_impl::admit_one(slot &s) {
   groups_run++;
   requests_run += group.size();
 
-  // enqueue: descriptors, staged inputs, the chain, staged outputs, completion
+  // enqueue: descriptors, staged inputs, the chain, staged outputs, completion.
+  // The group, its slot and its arena block are this thread's now, so the lock
+  // is not needed; submissions go on meanwhile (held, it made each of 24
+  // submissions wait for a group's 130 us of launches, and the groups small).
+  held.unlock();
   uint8_t *scratch = arena_base + offset;
   const std::vector<uint8_t> img = descriptor_image(best);
   cudaError_t e = cudaSuccess;
@@ -258,9 +262,10 @@ bool server_impl::admit_one(slot &s) {
     for (cudaStream_t fork : s.forks)
       cudaStreamSynchronize(fork);
     for (request *r : group)
-      r->status = e;
+      r->status = e; // read after done, which is set under the lock
     s.finished = true;
   }
+  held.lock();
   unsigned long long inflight = 0;
   for (auto &sl : slots)
     inflight += sl->busy;
@@ -292,7 +297,7 @@ void server_impl::run() {
     }
     // admissions, oldest request first
     for (auto &sp : slots)
-      if (!sp->busy && admit_one(*sp))
+      if (!sp->busy && admit_one(*sp, g))
         progress = true;
     bool busy = false;
     for (auto &sp : slots)
