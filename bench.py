@@ -720,7 +720,7 @@ def run_b200(args, dist: Dist) -> None:
     step_final_sum()
     line["final_sum"] = {"ms": round(time_steps(bc, stream, args.steps, step_final_sum), 4),
                          "what": "msm_b200_final_sum_async: sum 2^i R_i of the 254 results as one canonical affine point, on "
-                                 "the device (one block; latency-bound: 255 dependent doublings, 8 additions, one inversion)"}
+                                 "the device (a cluster of eight blocks; latency-bound: 142 dependent doublings, one inversion)"}
     bc.free(point_dev)
     extras = dist.rank == 0 and dist.world == 1
     if extras and not args.no_cpu_baseline:
