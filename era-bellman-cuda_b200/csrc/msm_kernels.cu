@@ -295,9 +295,8 @@ __global__ void __launch_bounds__(AFFINE_APPLY_THREADS, AFFINE_APPLY_MIN_BLOCKS)
 // Thread t takes warps [t E, (t + 1) E): its own product chain over their
 // totals (warp_inverse holds each one's prefix meanwhile), then the block's
 // products of the other threads' chains (warp_products within each warp, then
-// across the warps), one inversion of the block total by the binary extended
-// Euclidean algorithm, and the chain backwards.  The output counts are scanned
-// in the same arrangement.
+// across the warps), one inversion of the block total by division steps, and
+// the chain backwards.  The output counts are scanned in the same arrangement.
 __global__ void __launch_bounds__(AFFINE_INVERT_THREADS) affine_invert_kernel(const fe *__restrict__ warp_total, const uint32_t *__restrict__ warp_outputs,
                                                                               unsigned warps, fe *__restrict__ warp_inverse,
                                                                               unsigned long long *__restrict__ warp_base,
