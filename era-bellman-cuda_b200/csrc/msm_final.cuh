@@ -85,16 +85,16 @@ struct rns_stored {
 };
 
 struct rns_warp {
-  unsigned group, base; // of this lane: 0..2, its group's first lane
+  unsigned group, index; // of this lane: 0..2, and its residue 0..9
   rns::lane_table t;
 
   __device__ __forceinline__ rns_warp() {
     const unsigned lane = threadIdx.x & 31;
-    group = min(lane / rns::RESIDUES, rns::GROUPS - 1); // lanes 30, 31 repeat lanes 20, 21
-    base = group * rns::RESIDUES;
+    group = min(lane / rns::RESIDUES, rns::GROUPS - 1);
+    index = lane % rns::RESIDUES; // lanes 30 and 31 hold what lanes 20 and 21 hold: group 2, residues 0 and 1
     // every word through a volatile move: the table stays in registers instead
     // of being read again inside the doubling loop
-    const uint32_t *from = reinterpret_cast<const uint32_t *>(rns_tables.lane + lane % rns::RESIDUES);
+    const uint32_t *from = reinterpret_cast<const uint32_t *>(rns_tables.lane + index);
     uint32_t *to = reinterpret_cast<uint32_t *>(&t);
 #pragma unroll
     for (unsigned k = 0; k < sizeof(rns::lane_table) / 4; k++)
@@ -105,7 +105,7 @@ struct rns_warp {
 #endif
   }
   __device__ __forceinline__ auto extension() const {
-    return [first = base](int32_t v, auto sum) {
+    return [first = group * rns::RESIDUES](int32_t v, auto sum) {
 #pragma unroll
       for (int k = 0; k < (int)rns::RESIDUES; k++)
         sum(k, __shfl_sync(0xffffffffu, v, first + k));
@@ -116,7 +116,7 @@ struct rns_warp {
   }
   // group g's residues, in every lane
   __device__ __forceinline__ rns::residues from_group(const rns::residues &v, unsigned g) const {
-    const unsigned src = g * rns::RESIDUES + (threadIdx.x & 31) - base;
+    const unsigned src = g * rns::RESIDUES + index;
     return {__shfl_sync(0xffffffffu, v.a, src), __shfl_sync(0xffffffffu, v.b, src)};
   }
   __device__ __forceinline__ rns::residues pick(const rns::residues &g0, const rns::residues &g1, const rns::residues &g2) const {
@@ -185,15 +185,13 @@ struct rns_warp {
   __device__ __forceinline__ void put(rns_stored &to, const rns_point &p) const {
     const rns::residues z = from_group(p.z, 1);
     if ((threadIdx.x & 31) < rns::RESIDUES) {
-      const unsigned i = threadIdx.x & 31;
-      to.x[i] = p.x;
-      to.y[i] = p.y;
-      to.z[i] = z;
+      to.x[index] = p.x;
+      to.y[index] = p.y;
+      to.z[index] = z;
     }
   }
   __device__ __forceinline__ rns_point get(const rns_stored &from) const {
-    const unsigned i = (threadIdx.x & 31) - base;
-    return {from.x[i], from.y[i], from.z[i]};
+    return {from.x[index], from.y[index], from.z[index]};
   }
 
   // X, Y, Z as Montgomery-form field elements in (0, 2p), the same in every
@@ -202,8 +200,8 @@ struct rns_warp {
     const rns::residues leave = {t.leave_a, t.leave_b};
     const int64_t column = rns::product_column(t, pick(p.x, p.y, p.z), leave, extension());
     const unsigned lane = threadIdx.x & 31;
-    if (lane < rns::GROUPS * rns::RESIDUES && lane - base < 8)
-      columns[group][lane - base] = column;
+    if (lane < rns::GROUPS * rns::RESIDUES && index < 8)
+      columns[group][index] = column;
     __syncwarp();
     fe c; // lane g < 3 carries coordinate g
     int64_t carry = 0;
