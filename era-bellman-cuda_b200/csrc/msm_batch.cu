@@ -700,7 +700,7 @@ cudaError_t enqueue_batch(const batch_plan &b, uint8_t *scratch, cudaStream_t s,
     const uint8_t *gf = flags + grp.bucket_base;
     xyzz *const tree[2] = {reinterpret_cast<xyzz *>(at(grp.tree[0])), reinterpret_cast<xyzz *>(at(grp.tree[1]))};
     xyzz *const streams[2] = {reinterpret_cast<xyzz *>(at(grp.streams[0])), reinterpret_cast<xyzz *>(at(grp.streams[1]))};
-    CHECK(enqueue_window_sums(p, gb, gf, tree, streams, fs, launched));
+    CHECK(enqueue_window_sums(p, gb, gf, tree, streams, !forks, fs, launched));
     const unsigned level = tail_level(p.log_g);
     CHECK(launch_after(early, batch_reduce_tail_kernel, p.windows, TAIL_THREADS, tail_smem(p.log_g), fs, tree[level & 1], streams[level & 1], gb, gf,
                        reinterpret_cast<const unsigned *>(at(grp.members_dev)), p.c, p.log_m, p.log_g, level, io));

@@ -1,7 +1,5 @@
 // The final sum's kernel and entry point (msm_final.cuh has the method and the device code).
-#include "msm_device.cuh"
 #include "msm_final.cuh"
-#include "msm_host.cuh"
 #include "pointer_access.h"
 
 #include <cooperative_groups.h>
@@ -11,7 +9,6 @@ namespace msm_b200 {
 
 __global__ void __cluster_dims__(FINAL_BLOCKS, 1, 1) __launch_bounds__(FINAL_THREADS)
     final_sum_kernel(const jacobian *__restrict__ results, msm_b200_affine_point *point) {
-  begin_after_previous();
   __shared__ final_shared sh;
   final_sum_block(sh, cooperative_groups::this_cluster(), results, point);
 }
@@ -40,8 +37,8 @@ cudaError_t final_sum(const void *results, msm_b200_affine_point *point, cudaStr
     err = device_view(point, &p);
   if (err != cudaSuccess)
     return err;
-  return launch_after(early_launches(stream), final_sum_kernel, FINAL_BLOCKS, FINAL_THREADS, 0, stream, static_cast<const jacobian *>(r),
-                      static_cast<msm_b200_affine_point *>(p));
+  final_sum_kernel<<<FINAL_BLOCKS, FINAL_THREADS, 0, stream>>>(static_cast<const jacobian *>(r), static_cast<msm_b200_affine_point *>(p));
+  return cudaGetLastError();
 }
 
 } // namespace msm_b200

@@ -465,7 +465,9 @@ static cudaError_t enqueue_accumulation(const plan &p, const fe *scalars, const 
     // 1. digits (c <= 5: more windows than the digit kernel can count)
     const cleared_words counters = {zeros, (unsigned)((l.lookback_words - l.zeros) / 4)}; // zero counts .. work counter
     const cleared_words flag_words = {reinterpret_cast<uint32_t *>(flags), (unsigned)((slots + 3) / 4)};
-    CHECK(launch_after(p.early, digits_kernel, (n + 255) / 256, 256, 0, stream, scalars, n, p.c, p.windows, keys[0], vals[0], counters, flag_words));
+    // launched plainly: it is the call's first operation, or behind a chunk's copy event (see launch_after)
+    digits_kernel<<<(n + 255) / 256, 256, 0, stream>>>(scalars, n, p.c, p.windows, keys[0], vals[0], counters, flag_words);
+    CHECK(cudaGetLastError());
     m.launched++;
     CHECK(m.mark(stream));
     // 2. sort, 8 bits per pass: histogram, scan and scatter kernels
@@ -585,7 +587,7 @@ cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsign
 // of ACC_THREADS: at 2^22, blocks of 64 threads measured the same and blocks
 // of 96 slower (reduction 0.695 -> 0.815 ms).
 cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_t *flags, xyzz *const tree[2], xyzz *const streams[2],
-                                cudaStream_t stream, unsigned &launched) {
+                                bool behind_kernel, cudaStream_t stream, unsigned &launched) {
   // Launches with fewer jobs than one block of ACC_THREADS per SM run a group
   // of four lanes per job (msm_group4.cuh): there each job's chain of
   // additions is the launch's latency, and four times the threads still fit.
@@ -593,11 +595,11 @@ cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_
   auto blocks = [](unsigned long long threads) { return (unsigned)((threads + ACC_THREADS - 1) / ACC_THREADS); };
   const unsigned group_threads = p.windows << p.log_g;
   if (group_threads <= small)
-    CHECK(launch_after(p.early, reduce_groups_group4_kernel, blocks(4ull * group_threads), ACC_THREADS, 0, stream, buckets, flags, p.windows, p.log_b,
-                       p.log_m, tree[0], streams[0]));
+    CHECK(launch_after(p.early && behind_kernel, reduce_groups_group4_kernel, blocks(4ull * group_threads), ACC_THREADS, 0, stream, buckets, flags,
+                       p.windows, p.log_b, p.log_m, tree[0], streams[0]));
   else
-    CHECK(launch_after(p.early, reduce_groups_kernel, blocks(group_threads), ACC_THREADS, 0, stream, buckets, flags, p.windows, p.log_b, p.log_m,
-                       tree[0], streams[0]));
+    CHECK(launch_after(p.early && behind_kernel, reduce_groups_kernel, blocks(group_threads), ACC_THREADS, 0, stream, buckets, flags, p.windows,
+                       p.log_b, p.log_m, tree[0], streams[0]));
   launched++;
   for (unsigned level = 0; level < tail_level(p.log_g); level++) {
     const unsigned threads = p.windows * (level + 2) * ((1u << p.log_g) >> (level + 1));
@@ -617,7 +619,7 @@ static cudaError_t enqueue_reduction(const plan &p, const xyzz *buckets, const u
                                      cudaStream_t stream, stage_marks &m) {
   xyzz *const tree[2] = {reinterpret_cast<xyzz *>(scratch + l.tree[0]), reinterpret_cast<xyzz *>(scratch + l.tree[1])};
   xyzz *const streams[2] = {reinterpret_cast<xyzz *>(scratch + l.streams[0]), reinterpret_cast<xyzz *>(scratch + l.streams[1])};
-  CHECK(enqueue_window_sums(p, buckets, flags, tree, streams, stream, m.launched));
+  CHECK(enqueue_window_sums(p, buckets, flags, tree, streams, true, stream, m.launched));
   const unsigned level = tail_level(p.log_g);
   CHECK(launch_after(p.early, reduce_tail_kernel, p.windows, TAIL_THREADS, tail_smem(p.log_g), stream, tree[level & 1], streams[level & 1], buckets,
                      flags, p.c, p.log_m, p.log_g, level, results));

@@ -59,13 +59,20 @@ constexpr unsigned PROFILE_STAGES = 6;
 // Launches a kernel that begins with begin_after_previous().  With `early` its
 // blocks may be placed as soon as every block of the stream's previous kernel
 // has ended (programmatic stream serialization without an explicit trigger),
-// so the launch and the flush between two kernels overlap: MSM at 2^8 points
-// 0.134 -> 0.110 ms (11 kernels), 2^12 0.171 -> 0.146, 200,003 skewed 0.582 ->
-// 0.532, 2^18 1.110 -> 1.057, 2^22 10.802 -> 10.748.  Kernels that let the next
-// one start at their own start (griddepcontrol.launch_dependents) were slower,
-// 2^12 0.198 and 2^18 1.185 ms: the next kernel's blocks then pile up on the
-// SMs that are free at that moment.  A batch that is captured records plain
-// kernels: its graph took the same time either way (2.702 against 2.706 ms).
+// so the launch and the flush between two kernels overlap.  For every kernel of
+// a call: MSM at 2^8 points 0.134 -> 0.110 ms (11 kernels), 2^12 0.171 -> 0.146,
+// 200,003 skewed 0.582 -> 0.532, 2^18 1.110 -> 1.057, 2^22 10.802 -> 10.748.
+// Only behind another kernel (or memset) of the same call, though: the wait
+// covers the kernel before, not what that one should itself have waited for.
+// So a call's first kernel is launched plainly, because the caller's last one
+// may have been launched early and have ended without waiting, and so is one
+// behind a wait for another stream's event.  That gives back 4 to 6 us of an
+// MSM with its final sum (two calls; 2^18 points 1,241 -> 1,249 us).
+// Kernels that let the next one start at their own start
+// (griddepcontrol.launch_dependents) were slower, 2^12 0.198 and 2^18 1.185 ms:
+// the next kernel's blocks then pile up on the SMs that are free at that
+// moment.  A batch that is captured records plain kernels: its graph took the
+// same time either way (2.702 against 2.706 ms).
 template <class... P, class... A>
 cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchAttribute attribute{};
@@ -96,8 +103,10 @@ inline bool early_launches(cudaStream_t stream) {
 // reduce_level_kernel per level) for the p.windows windows of 2^(c-1) bucket
 // slots at `buckets`; afterwards streams[p.log_g & 1] holds each window's sums
 // for the gather kernels.  tree / streams: the ping-pong buffers of the plan.
+// behind_kernel: the stream's last operation is a kernel of the same call (see
+// launch_after).
 cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_t *flags, xyzz *const tree[2], xyzz *const streams[2],
-                                cudaStream_t stream, unsigned &launched);
+                                bool behind_kernel, cudaStream_t stream, unsigned &launched);
 // Folds `heads` head partial sums (hb[0], hp[0]; one bucket's heads
 // contiguous) into their buckets, level by level, ping-ponging hb / hp.
 cudaError_t enqueue_merge_heads(uint32_t *const hb[2], xyzz *const hp[2], unsigned heads, xyzz *buckets, unsigned sms, bool early, cudaStream_t stream,

@@ -9,7 +9,6 @@ namespace msm_b200 {
 __global__ void __launch_bounds__(256) digits_kernel(const fe *__restrict__ scalars, unsigned n, unsigned c, unsigned windows,
                                                      uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, cleared_words first,
                                                      cleared_words second) {
-  begin_after_previous();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   for (unsigned k = i; k < first.count; k += gridDim.x * blockDim.x)
     first.at[k] = 0;
