@@ -15,6 +15,7 @@
 // one host clock.
 #include "bellman-cuda-b200.h"
 #include "device_arena.h"
+#include "fork_set.h"
 #include "msm_batch.cuh"
 
 #include <algorithm>
@@ -55,10 +56,8 @@ struct slot {
   cudaStream_t stream = nullptr;
   uint8_t *staging = nullptr; // pinned host copy of the group's descriptors
   size_t staging_bytes = 0;
-  // for the group's reductions, one chain per window width, side by side (as
-  // many as any group of this slot has needed; a width each at most)
-  std::vector<cudaStream_t> forks;
-  std::vector<cudaEvent_t> fork_events;
+  // for the group's reductions, one chain per window width, side by side
+  fork_set<cudaStream_t, cudaEvent_t> forks;
   bool busy = false;
   // Set by the completion host function, which must never wait for the
   // server lock: the scheduler makes CUDA calls while holding it, and some of
@@ -66,23 +65,16 @@ struct slot {
   std::atomic<bool> finished{false};
   std::vector<request *> members;
   size_t arena_offset = 0, arena_bytes = 0;
-
-  // at least `groups` fork streams and one event more
-  cudaError_t reserve_forks(size_t groups) {
-    cudaError_t e = cudaSuccess;
-    while (e == cudaSuccess && forks.size() < groups) {
-      cudaStream_t fork = nullptr;
-      if ((e = cudaStreamCreateWithFlags(&fork, cudaStreamNonBlocking)) == cudaSuccess)
-        forks.push_back(fork);
-    }
-    while (e == cudaSuccess && fork_events.size() < groups + 1) {
-      cudaEvent_t event = nullptr;
-      if ((e = cudaEventCreateWithFlags(&event, cudaEventDisableTiming)) == cudaSuccess)
-        fork_events.push_back(event);
-    }
-    return e;
-  }
 };
+
+// one chain per width of the table, as far as its streams can be had
+void create_forks(slot &s, size_t widths) {
+  auto made = [](cudaError_t e) { return e == cudaSuccess ? true : (cudaGetLastError(), false); };
+  if (widths > 1)
+    s.forks.create(
+        widths, [&](cudaStream_t &stream) { return made(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); },
+        [&](cudaEvent_t &event) { return made(cudaEventCreateWithFlags(&event, cudaEventDisableTiming)); });
+}
 
 struct server_impl {
   int device = 0, sms = 0;
@@ -248,10 +240,9 @@ bool server_impl::admit_one(slot &s, std::unique_lock<std::mutex> &held) {
   }
   if (e == cudaSuccess)
     e = enqueue_io(reinterpret_cast<batch_io *>(scratch + best.io), best.instances, scalars.data(), results.data(), s.stream);
+  const bool forked = s.forks.serves(best.groups.size()); // otherwise the chains follow one another
   if (e == cudaSuccess)
-    e = s.reserve_forks(best.groups.size());
-  if (e == cudaSuccess)
-    e = enqueue_batch(best, scratch, s.stream, s.forks.data(), s.fork_events.data(), true, nullptr);
+    e = enqueue_batch(best, scratch, s.stream, forked ? s.forks.streams.data() : nullptr, forked ? s.forks.events.data() : nullptr, true, nullptr);
   for (size_t k = 0; k < group.size() && e == cudaSuccess; k++)
     if (group[k]->host_results)
       e = cudaMemcpyAsync(group[k]->results, results[k], RESULT_BITS * sizeof(jacobian), cudaMemcpyDeviceToHost, s.stream);
@@ -260,7 +251,7 @@ bool server_impl::admit_one(slot &s, std::unique_lock<std::mutex> &held) {
   if (e != cudaSuccess) {
     // nothing more is enqueued for this group: wait for what was, then fail it
     cudaStreamSynchronize(s.stream);
-    for (cudaStream_t fork : s.forks)
+    for (cudaStream_t fork : s.forks.streams)
       cudaStreamSynchronize(fork);
     for (request *r : group)
       r->status = e; // read after done, which is set under the lock
@@ -323,9 +314,9 @@ server_impl::~server_impl() {
       cudaStreamSynchronize(sp->stream);
       cudaStreamDestroy(sp->stream);
     }
-    for (cudaStream_t fork : sp->forks)
+    for (cudaStream_t fork : sp->forks.streams)
       cudaStreamDestroy(fork);
-    for (cudaEvent_t event : sp->fork_events)
+    for (cudaEvent_t event : sp->forks.events)
       cudaEventDestroy(event);
     if (sp->staging)
       cudaFreeHost(sp->staging);
@@ -358,6 +349,7 @@ cudaError_t server_create(server_impl **out, const base_table_impl *table, size_
   if (e != cudaSuccess)
     return e;
   srv->arena.reset(scratch_budget);
+  const size_t widths = MAX_TABLE_BITS + 1 - std::count(std::begin(table->mult), std::end(table->mult), nullptr);
   for (unsigned k = 0; k < streams; k++) {
     std::unique_ptr<slot> s(new (std::nothrow) slot);
     if (!s)
@@ -365,6 +357,7 @@ cudaError_t server_create(server_impl **out, const base_table_impl *table, size_
     s->server = srv.get();
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess)
       return e;
+    create_forks(*s, std::min<size_t>(widths, max_group));
     srv->slots.push_back(std::move(s));
   }
   srv->scheduler = std::thread([p = srv.get()] { p->run(); });
