@@ -170,3 +170,71 @@ def test_server_poisson_arrivals(env, oracle):
         assert oracle.horner(b.results()) == oracle.msm_checksum(env.k[: len(s)], s), f"request {j}"
         b.free()
     bc.server_destroy(server)
+
+
+def test_server_many_threads(env, oracle):
+    """Six threads submit and wait while groups are being planned and enqueued,
+    two more read the statistics and submit requests that can never fit.  Every
+    point is right, the counts never run backwards or past what was submitted,
+    and nothing is left held."""
+    bc = env.bc
+    threads, each = 6, 8
+    reqs = make_requests(threads * each, 15, lo=8, hi=15)
+    bufs = [Buffers(bc, s, j) for j, s in enumerate(reqs)]
+    big = synth.uniform_scalars(78, 1 << 18)
+    big_buf = Buffers(bc, big, 0)
+    server = bc.server_create(env.table, 48 << 20, streams=3, max_group=8)
+    out, errors, running = [None] * len(reqs), [], [threads]
+    lock = threading.Lock()
+
+    def guarded(body):
+        def run(*args):
+            try:
+                body(*args)
+            except Exception as e:  # reported below, on the main thread
+                errors.append(e)
+        return run
+
+    @guarded
+    def client(t):
+        try:
+            mine = range(t, len(reqs), threads)
+            for half in (list(mine)[:each // 2], list(mine)[each // 2:]):
+                tickets = [(j, bc.server_submit(server, bufs[j].s, len(reqs[j]), bufs[j].r)) for j in half]
+                for j, ticket in tickets:
+                    rc, times = bc.server_wait(server, ticket)
+                    assert rc == 0 and times.submit_us <= times.start_us <= times.done_us
+                    out[j] = bufs[j].results()
+        finally:
+            with lock:
+                running[0] -= 1
+
+    @guarded
+    def reader():
+        last = 0
+        while running[0]:
+            stats = bc.server_stats(server)
+            assert last <= stats.requests <= len(reqs) and stats.groups <= stats.requests
+            assert stats.arena_used <= stats.arena_bytes and stats.max_inflight_groups <= 3
+            last = stats.requests
+
+    @guarded
+    def refused():
+        for _ in range(4):
+            rc, _ = bc.server_wait(server, bc.server_submit(server, big_buf.s, len(big), big_buf.r))
+            assert rc == env.bcm.BC_ERROR_MEMORY_ALLOCATION
+
+    workers = [threading.Thread(target=client, args=(t,)) for t in range(threads)]
+    workers += [threading.Thread(target=reader), threading.Thread(target=refused)]
+    for w in workers:
+        w.start()
+    for w in workers:
+        w.join()
+    assert not errors, errors
+    stats = bc.server_stats(server)
+    assert stats.requests == len(reqs) and stats.pending == 0 and stats.arena_used == 0
+    bc.server_destroy(server)
+    for j, (b, s) in enumerate(zip(bufs, reqs)):
+        assert oracle.horner(out[j]) == oracle.msm_checksum(env.k[: len(s)], s), f"request {j}"
+        b.free()
+    big_buf.free()
