@@ -735,7 +735,7 @@ template <class F> struct field {
     return (int32_t)((low * F::INV) << 2) >> 2;
   }
 
-  // Thirty division steps (see inverse_binary) on the low words of f and g:
+  // Thirty division steps (see inverse_standard) on the low words of f and g:
   // the new (f, g) is the matrix ((u, v), (q, r)) times the old, / 2^30.
   struct steps30 {
     int32_t u, v, q, r;
@@ -804,10 +804,12 @@ template <class F> struct field {
 
   // a^-1 mod m for a canonical a in standard (not Montgomery) form, by the
   // division steps of D. J. Bernstein and B.-Y. Yang ("Fast constant-time gcd
-  // computation and modular inversion", TCHES 2019), in the form that starts
-  // from delta = 1/2, for which 590 steps end every 256-bit input.  One step
-  // on an odd f and any g: (f, g) becomes (g, -f) first when delta > 0 and g
-  // is odd, then g + f if g is odd, then g / 2.  Thirty steps depend on the
+  // computation and modular inversion", TCHES 2019).  The start at delta = 1/2,
+  // with its bound of 590 steps for every 256-bit input, and the layout of
+  // thirty steps a round on nine signed 30-bit words are those that P. Wuille
+  // describes in "The safegcd implementation in libsecp256k1 explained".  One
+  // step on an odd f and any g: (f, g) becomes (g, -f) first when delta > 0 and
+  // g is odd, then g + f if g is odd, then g / 2.  Thirty steps depend on the
   // low words alone, so they run on two 32-bit registers and collect a 2 x 2
   // matrix, which is then applied to f, g and, modulo m, to d, e, for which
   // f = d a and g = e a (mod m) stays true; d and e grow by at most m / 2 a
@@ -816,7 +818,7 @@ template <class F> struct field {
   // lanes (inverse_group4), against 100,191 for the binary extended Euclidean
   // algorithm (Hankerson, Menezes and Vanstone, Algorithm 2.22), whose halvings
   // each touch all words.  0 gives 0.
-  static BN_HD fe inverse_binary(const fe &a) {
+  static BN_HD fe inverse_standard(const fe &a) {
     if (is_zero_exact(a))
       return zero();
     int32_t f[INV_WORDS], g[INV_WORDS], d[INV_WORDS], e[INV_WORDS];
@@ -852,19 +854,6 @@ template <class F> struct field {
     }
     // g = 0 and f = +-1 = d a: the inverse is +-d, |d| < 11 m
     return join30(d, f[INV_WORDS - 1] < 0 ? -1 : 1);
-  }
-
-  // exponentiation by m - 2 (Fermat inverse), Montgomery domain; 0 -> 0
-  static BN_HD fe inverse(const fe &a) {
-    fe e = modulus();
-    e.l[0] -= 2; // m is odd and > 2, no borrow
-    fe acc = one();
-    for (int i = 255; i >= 0; i--) {
-      acc = sqr(acc);
-      if ((e.l[i >> 5] >> (i & 31)) & 1)
-        acc = mul(acc, a);
-    }
-    return acc;
   }
 };
 

@@ -128,7 +128,7 @@ __device__ __forceinline__ xyzz add_group4(const xyzz &p, const xyzz &q) {
   return r;
 }
 
-// fq::inverse_binary shared by a group of four lanes (a standard-form
+// fq::inverse_standard shared by a group of four lanes (a standard-form
 // canonical value, the same in all four): the 30 division steps run in every
 // lane, and of the four rows that the matrix is applied to (d and e modulo p,
 // f and g) each lane computes one and swaps it with its neighbour's.  Lanes 0

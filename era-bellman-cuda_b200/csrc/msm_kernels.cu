@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(AFFINE_INVERT_THREADS) affine_invert_kernel(co
     if (lane == WARPS - 1)
       *count_out = ci;
     if (lane == 0)
-      s_inverse = fq::to_mont(fq::inverse_binary(fq::from_mont(all)));
+      s_inverse = fq::to_mont(fq::inverse_standard(fq::from_mont(all)));
   }
   __syncthreads();
   fe inv = fq::mul(fq::mul(s_inverse, s_others[wid]), others);

@@ -16,7 +16,8 @@ template <class T> static void st(uint32_t *w, const T &t) { std::memcpy(w, &t, 
 
 extern "C" {
 
-// op: 0 mul, 1 sqr, 2 add, 3 sub, 4 neg, 5 reduce_full, 6 from_mont, 7 to_mont, 8 inverse, 9 dbl
+// op: 0 mul, 1 sqr, 2 add, 3 sub, 4 neg, 5 reduce_full, 6 from_mont, 7 to_mont, 8 inverse in
+// Montgomery form (as curve::to_affine takes it), 9 dbl, 10 neg_nonzero, 11 inverse in standard form
 void fc_fq_op(int op, const uint32_t *a, const uint32_t *b, uint32_t *out, int n) {
   for (int i = 0; i < n; i++) {
     const fe x = ld<fe>(a + 8 * i), y = ld<fe>(b + 8 * i);
@@ -30,10 +31,10 @@ void fc_fq_op(int op, const uint32_t *a, const uint32_t *b, uint32_t *out, int n
     case 5: r = fq::reduce_full(x); break;
     case 6: r = fq::from_mont(x); break;
     case 7: r = fq::to_mont(x); break;
-    case 8: r = fq::inverse(x); break;
+    case 8: r = fq::to_mont(fq::inverse_standard(fq::from_mont(x))); break;
     case 9: r = fq::dbl(x); break;
     case 10: r = fq::neg_nonzero(x); break;
-    case 11: r = fq::inverse_binary(x); break;
+    case 11: r = fq::inverse_standard(x); break;
     }
     st(out + 8 * i, r);
   }
@@ -88,11 +89,15 @@ void fc_from_affine(const uint32_t *a, uint32_t *out) { st(out, curve::from_affi
 void fc_to_jacobian(const uint32_t *p, uint32_t *out) { st(out, curve::to_jacobian(ld<xyzz>(p))); }
 void fc_from_jacobian(const uint32_t *p, uint32_t *out) { st(out, curve::from_jacobian(ld<jacobian>(p))); }
 int fc_to_affine_standard(const uint32_t *p, uint32_t *out) {
-  fe x, y;
-  const bool inf = curve::to_affine_standard(ld<xyzz>(p), x, y);
-  st(out, x);
-  st(out + 8, y);
-  return inf ? 1 : 0;
+  const xyzz point = ld<xyzz>(p);
+  if (curve::is_inf(point)) {
+    std::memset(out, 0, 64);
+    return 1;
+  }
+  const affine a = curve::to_affine(point);
+  st(out, fq::from_mont(a.x));
+  st(out + 8, fq::from_mont(a.y));
+  return 0;
 }
 void fc_infinity(uint32_t *out) { st(out, curve::infinity()); }
 

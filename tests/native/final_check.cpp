@@ -5,12 +5,16 @@
 //                                        per sum -> 20 words each
 //   final_check lanes IN OUT             pairs of Jacobian points -> per lane
 //                                        the residues after each warp operation
+//   final_check inverse IN OUT           values (8 words each, a multiple of
+//                                        eight of them) -> their inverses, a
+//                                        group of four lanes each
 #include "warp_emulation.h"
 
 #include "msm_final.cuh"
 
 #include <fstream>
 #include <iterator>
+#include <string>
 
 using namespace msm_b200;
 
@@ -92,12 +96,31 @@ std::vector<uint32_t> lanes(const std::vector<uint32_t> &in) {
   return out;
 }
 
+std::vector<uint32_t> inverses(const std::vector<uint32_t> &in) {
+  std::vector<uint32_t> out(in.size());
+  for (size_t k = 0; k + 64 <= in.size(); k += 64)
+    emulation::run(1, 32, false, [&](unsigned) {
+      const unsigned lane = threadIdx.x;
+      fe a;
+      std::memcpy(&a, in.data() + k + lane / 4 * 8, sizeof(a));
+      const fe r = inverse_group4(a);
+      fe first;
+      for (int i = 0; i < 8; i++)
+        first.l[i] = __shfl_sync(0xffffffffu, r.l[i], lane & 28);
+      if (std::memcmp(&first, &r, sizeof(r)) != 0)
+        emulation::fail("a group's lanes differ", "inverse_group4");
+      std::memcpy(out.data() + k + lane / 4 * 8, &r, sizeof(r));
+    });
+  return out;
+}
+
 } // namespace
 
 int main(int argc, char **argv) {
   if (argc < 4)
     return 2;
   const std::vector<uint32_t> in = read_words(argv[2]);
-  write_words(argv[3], std::strcmp(argv[1], "sum") == 0 ? sums(in, argc > 4) : lanes(in));
+  const std::string mode = argv[1];
+  write_words(argv[3], mode == "sum" ? sums(in, argc > 4) : mode == "lanes" ? lanes(in) : inverses(in));
   return 0;
 }

@@ -81,8 +81,9 @@ def test_fq_inverse(field_check):
 
 
 def test_fq_inverse_binary(field_check):
-    """Binary extended-Euclid inverse of canonical standard-form values
-    (the on-device final reduction's inversion): a * a^-1 = 1 mod p, 0 -> 0."""
+    """Inverse of canonical standard-form values by division steps (the affine
+    conversions' inversion; the final sum shares one between four lanes, see
+    test_final_sum_model.py): a * a^-1 = 1 mod p, 0 -> 0."""
     rng = np.random.Generator(np.random.PCG64(12))
     xs = [int.from_bytes(rng.bytes(32), "little") % P for _ in range(2000)]
     xs += [0, 1, 2, 3, P - 1, P - 2, P // 2, (P + 1) // 2, 1 << 128, (1 << 253) - 1, 0xFFFFFFFF, 1 << 32]
@@ -209,8 +210,9 @@ def test_square_matches_cios(field_check, pairs):
 
 
 def test_jacobian_round_trip_and_standard_affine(field_check, oracle):
-    """from_jacobian / to_affine_standard (the final-sum kernel's input and
-    output conversions): Jacobian points with random Z, infinity with Z = 0."""
+    """from_jacobian (the final sum's input conversion) and to_affine (the base
+    tables'), its coordinates taken out of Montgomery form: Jacobian points with
+    random Z, infinity with Z = 0."""
     table = H.load_g_bases()
     f = field_check
     rng = np.random.Generator(np.random.PCG64(13))

@@ -116,3 +116,14 @@ def test_lanes_of_a_warp(check):
             groups = lanes[:GROUPS * RESIDUES].reshape(GROUPS, RESIDUES, 6)
             assert (groups[:, :, :4] == groups[0, :, :4]).all(), name
             assert (groups[1, :, 4:] == groups[2, :, 4:]).all(), name
+
+
+def test_inverse_of_a_group(check):
+    """inverse_group4 on edge values and random ones, groups of one warp ending
+    after different numbers of rounds: a a^-1 = 1 modulo p, 0 -> 0."""
+    rng = np.random.Generator(np.random.PCG64(12))
+    values = [0, 1, 2, 3, P - 1, P - 2, P // 2, (P + 1) // 2, 1 << 128, (1 << 253) - 1, 0xFFFFFFFF, 1 << 32, 1 << 30, (1 << 30) - 1, P - (1 << 30), 0]
+    values += [int.from_bytes(rng.bytes(32), "little") % P for _ in range(400)]
+    out = check("inverse", np.concatenate([H.limbs(v) for v in values])).reshape(-1, 8)
+    for v, r in zip(values, out):
+        assert H.to_int(r) == (pow(v, -1, P) if v else 0), hex(v)
