@@ -809,20 +809,6 @@ __device__ __forceinline__ void accumulate_range(const SEG &seg, const uint32_t 
   }
 }
 
-// How many of the `ranges` hold entries, for a list of `total`: with more than
-// one range per thread, only as many as there are threads when the list is too
-// short to give each ACC_MIN_ENTRIES.  The host plans the ranges for lists
-// without zero digits; how many entries are left is known here.  Measured with
-// 75,776 threads and one / two ranges each: 2^22 skewed points (14.3 M of 62.9 M
-// entries left, 189 / 94 per range) 3.458 / 3.617 ms, a 2.5 M-point chunk (495 /
-// 247 per range) 8.97 / 8.70 ms end to end, 2^22 uniform (830 / 415) 11.31 /
-// 10.74 ms, 2^20 (220 / 110) 3.29 / 3.47 ms.
-__device__ __forceinline__ unsigned long long active_ranges(unsigned long long total, unsigned ranges) {
-  const unsigned threads = gridDim.x * ACC_THREADS;
-  const unsigned long long most = ranges > threads && total < (unsigned long long)ranges * ACC_MIN_ENTRIES ? threads : ranges;
-  return min(total, most);
-}
-
 // The work loop over all ranges (see accumulate_range).  Only the first
 // active_ranges(M, ranges) ranges hold entries, so every active range holds at
 // least one entry and the heads of one bucket stay contiguous (an empty range
@@ -834,7 +820,7 @@ __device__ __forceinline__ void accumulate_ranges(const SEG &seg, const uint32_t
                                                   uint8_t *__restrict__ flags, uint32_t *__restrict__ head_bucket, xyzz *__restrict__ head_point,
                                                   uint4 (*s_base)[4][ACC_THREADS]) {
   const unsigned long long total = seg.prefix(seg.count());
-  const unsigned long long active = active_ranges(total, ranges);
+  const unsigned long long active = active_ranges(total, ranges, gridDim.x * ACC_THREADS);
   const unsigned lane = threadIdx.x & 31;
   for (;;) {
     unsigned first = 0;

@@ -119,13 +119,12 @@ static device_info get_device_info(int device) {
 
 // Accumulation ranges: a whole number k <= per_thread of ranges per thread,
 // as large as keeps ACC_MIN_ENTRIES entries per range (a range's start-up --
-// cursor search, first gather, head -- costs about as much as a few hundred
-// additions: 2^21 points ran 3 % slower with 205-entry ranges than with 410).
-// Whole multiples keep every warp at the same number of rounds.  Measured at
-// the 3.5M-point second chunk of a host-input 2^22 MSM (52 M entries): two
-// ranges of 346 entries per thread beat one of 692 by 0.48 ms (end to end
-// 12.90 -> 12.40 ms), and at the 2.5M-point chunk of 3,000,017 points two of
-// 247 beat one of 495 by 0.27 ms, hence 240.
+// cursor search, first gather, head -- costs about as much as some hundred
+// additions).  Whole multiples keep every warp at the same number of rounds.
+// Measured at both sides of the line: see active_ranges; end to end, the
+// 3.5M-point second chunk of a host-input 2^22 MSM (52 M entries) takes 0.48 ms
+// less with two ranges of 346 entries per thread than with one of 692 (12.90 ->
+// 12.40 ms), the 2.5M-point chunk of 3,000,017 points 0.27 ms less with two of 247.
 unsigned accumulation_ranges(unsigned threads, unsigned long long entries, unsigned per_thread) {
   const unsigned long long fit = entries / ((unsigned long long)threads * ACC_MIN_ENTRIES);
   const unsigned long long k = std::max(1ull, std::min((unsigned long long)per_thread, fit));

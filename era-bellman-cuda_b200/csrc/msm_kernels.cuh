@@ -80,6 +80,21 @@ template <unsigned THREADS, unsigned ITEMS> constexpr size_t lookback_smem_bytes
 constexpr unsigned ACC_THREADS = 128;
 constexpr unsigned ACC_MIN_ENTRIES = 240; // per accumulation range, when a thread has several (see active_ranges)
 
+// How many of an accumulation's `ranges` hold entries, for a list of `total`:
+// with more than one range per thread, only as many as there are threads when
+// the list is too short to give each ACC_MIN_ENTRIES.  The host plans the ranges
+// for lists without zero digits; how many entries are left is known on the
+// device.  Measured with 75,776 threads and one / two ranges each: 2^20 points
+// (220 / 110 entries per range) 3.29 / 3.47 ms, 2^22 skewed (14.3 M of 62.9 M
+// entries left, 189 / 94) 3.458 / 3.617 ms, 1.95 M (386 / 193) 5.61 / 5.91, 2.05
+// M (406 / 203) 5.87 / 5.60, 2.35 M (465 / 233) 6.63 / 6.32, 2.85 M (564 / 282)
+// 7.91 / 7.54, 2^22 (830 / 415) 11.31 / 10.74; between 173 and 183 entries two
+// ranges were the faster ones too (1.75 M points 5.11 / 4.88).
+__host__ __device__ constexpr unsigned long long active_ranges(unsigned long long total, unsigned ranges, unsigned threads) {
+  const unsigned long long most = ranges > threads && total < (unsigned long long)ranges * ACC_MIN_ENTRIES ? threads : ranges;
+  return total < most ? total : most;
+}
+
 // Window w's entries start at w * window_stride(n): n rounded up to 32
 // entries, so that every window segment starts on a 128-byte line and the
 // digit kernels' stores stay whole lines whatever n is (at n = 3,495,254

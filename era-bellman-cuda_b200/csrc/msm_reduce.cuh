@@ -3,7 +3,6 @@
 // one after another in shared memory, then the window's results.
 #pragma once
 
-#include "msm_device.cuh"
 #include "msm_group4.cuh"
 
 namespace msm_b200 {

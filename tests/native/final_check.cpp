@@ -5,6 +5,8 @@
 //                                        per sum -> 20 words each
 //   final_check lanes IN OUT             pairs of Jacobian points -> per lane
 //                                        the residues after each warp operation
+//   final_check constants IN OUT         per split group a, b (4 words each) and
+//                                        their signs, then beta (IN is not read)
 //   final_check inverse IN OUT           values (8 words each, a multiple of
 //                                        eight of them) -> their inverses, a
 //                                        group of four lanes each
@@ -96,6 +98,19 @@ std::vector<uint32_t> lanes(const std::vector<uint32_t> &in) {
   return out;
 }
 
+std::vector<uint32_t> constants() {
+  std::vector<uint32_t> out;
+  for (const split_power &p : split_powers) {
+    out.insert(out.end(), p.a, p.a + 4);
+    out.insert(out.end(), p.b, p.b + 4);
+    out.push_back(p.a_negative);
+    out.push_back(p.b_negative);
+  }
+  const fe beta = endomorphism_beta();
+  out.insert(out.end(), beta.l, beta.l + 8);
+  return out;
+}
+
 std::vector<uint32_t> inverses(const std::vector<uint32_t> &in) {
   std::vector<uint32_t> out(in.size());
   for (size_t k = 0; k + 64 <= in.size(); k += 64)
@@ -121,6 +136,6 @@ int main(int argc, char **argv) {
     return 2;
   const std::vector<uint32_t> in = read_words(argv[2]);
   const std::string mode = argv[1];
-  write_words(argv[3], mode == "sum" ? sums(in, argc > 4) : mode == "lanes" ? lanes(in) : inverses(in));
+  write_words(argv[3], mode == "sum" ? sums(in, argc > 4) : mode == "lanes" ? lanes(in) : mode == "constants" ? constants() : inverses(in));
   return 0;
 }

@@ -127,3 +127,19 @@ def test_inverse_of_a_group(check):
     out = check("inverse", np.concatenate([H.limbs(v) for v in values])).reshape(-1, 8)
     for v, r in zip(values, out):
         assert H.to_int(r) == (pow(v, -1, P) if v else 0), hex(v)
+
+
+def test_split_constants(check, oracle):
+    """beta and lambda are the endomorphism's: phi(G) = (beta x, y) = lambda G; and
+    every split power is 2^(16 g) with both halves below 2^126, the bits summed."""
+    lam = 0xB3C4D79D41A917585BFC41088D8DAAA78B17EA66B99C90DD
+    out = check("constants", np.zeros(0))
+    beta = H.to_int(out[-8:]) * pow(MONT, -1, P) % P
+    assert beta != 1 and pow(beta, 3, P) == 1 and (lam * lam + lam + 1) % H.R == 0
+    for x, y in H.load_g_bases()[:3]:
+        assert oracle.affine_mul(x, y, lam) == (False, beta * x % P, y)
+    rows = out[:-8].reshape(8, 10)
+    for g, row in zip(range(8, 16), rows):
+        a, b = H.to_int(row[:4]), H.to_int(row[4:8])
+        assert a < 1 << 126 and b < 1 << 126
+        assert ((-a if row[8] else a) + (-b if row[9] else b) * lam - (1 << (16 * g))) % H.R == 0

@@ -194,33 +194,75 @@ def test_model_matches_sum(trial):
     assert model_msm(scal, kl, c, T) == sum(s * k for s, k in zip(scal, kl)) % R
 
 
-def model_final_sum(values, threads=128, result_bits=254):
-    """The index arithmetic of final_sum_kernel (msm_final.cu) with points as
-    integers mod R (doubling = 2x, addition = x + y): level 0 per thread
-    (R_2t + 2 R_2t+1), level 1 per even thread (partner doubled twice),
-    levels 2..7 per group of four lanes, group g adding part[g 2^L + 2^(L-1)]
-    doubled 2^L times into part[g 2^L].  Every partner index must stay in
-    the block and be read before anyone writes it at that level."""
-    part = [0] * threads
-    for t in range(threads):
-        if 2 * t + 1 < result_bits:
-            part[t] = (values[2 * t] + 2 * values[2 * t + 1]) % R
-    for t in range(0, threads, 2):
-        part[t] = (part[t] + 4 * part[t + 1]) % R
-    level = 2
-    while (1 << level) <= threads:
-        pairs = threads >> level
-        targets, partners = set(), set()
-        for group in range(threads // 4):
-            if group < pairs:
-                target, partner = group << level, (group << level) + (1 << (level - 1))
-                assert partner < threads
-                targets.add(target)
-                partners.add(partner)
-                part[target] = (part[target] + pow(2, 1 << level, R) * part[partner]) % R
-        assert not targets & partners  # no group reads a slot another group writes
-        level += 1
-    return part[0]
+def split(multiplier):
+    """(a, b) with a + b lambda = multiplier mod R, |a|, |b| < 2^127: rounded
+    multiples of a short basis of {(a, b): a + b lambda = 0}."""
+    (a1, b1), (a2, b2) = LATTICE
+    det = a1 * b2 - a2 * b1
+    nearest = lambda x: (2 * x + det) // (2 * det)
+    k1, k2 = nearest(multiplier * b2), nearest(-multiplier * b1)
+    return multiplier - k1 * a1 - k2 * a2, -k1 * b1 - k2 * b2
+
+
+def short_basis():
+    """Two short vectors of that lattice, from the extended Euclidean algorithm
+    on R and lambda stopped around the square root of R."""
+    rows = [(R, 0), (LAMBDA, 1)]  # (r, t) with r = t lambda mod R
+    while rows[-1][0] >= 1 << 127:
+        q = rows[-2][0] // rows[-1][0]
+        rows.append((rows[-2][0] - q * rows[-1][0], rows[-2][1] - q * rows[-1][1]))
+    q = rows[-2][0] // rows[-1][0]
+    after = (rows[-2][0] - q * rows[-1][0], rows[-2][1] - q * rows[-1][1])
+    before = min(rows[-2], after, key=lambda v: v[0] ** 2 + v[1] ** 2)
+    return (rows[-1][0], -rows[-1][1]), (before[0], -before[1])
+
+
+LAMBDA = 0xB3C4D79D41A917585BFC41088D8DAAA78B17EA66B99C90DD
+LATTICE = short_basis()
+
+
+def model_final_sum(values, blocks=8, parts=16, result_bits=254):
+    """The steps of the final sum (msm_final.cuh) with points as integers mod R
+    (doubling = 2x, addition = x + y, phi = lambda x): every block's 16 pairs
+    and its two groups' levels, the split of the upper eight groups, the digit
+    sums Q_j of 16 bits j per block, the blocks' levels over those bits and the
+    last three over the blocks.  No partner of a level may be another target."""
+    part = [[0] * parts for _ in range(blocks)]
+
+    def level(p, level, doublings):
+        targets = range(0, parts, 1 << level)
+        partners = [t + (1 << (level - 1)) for t in targets]
+        assert max(partners) < parts and not set(targets) & set(partners)
+        for t, o in zip(targets, partners):
+            p[t] = (p[t] + pow(2, doublings, R) * p[o]) % R
+
+    for k in range(blocks):
+        for pair in range(parts):
+            r = 2 * (k * parts + pair)
+            if r + 1 < result_bits:
+                part[k][pair] = (values[r] + 2 * values[r + 1]) % R
+        for lv in (1, 2, 3):
+            level(part[k], lv, 1 << lv)
+    group = [part[g // 2][(g & 1) * (parts // 2)] for g in range(2 * blocks)]
+    digits = {g: split(1 << (16 * g)) for g in range(8, 16)}
+    for k in range(blocks):
+        for bit in range(parts):
+            j = parts * k + bit
+            q = group[k] if bit == 0 else 0
+            for g, halves in digits.items():
+                for half, point in zip(halves, (group[g], LAMBDA * group[g])):
+                    assert abs(half) < 1 << (blocks * parts)
+                    if abs(half) >> j & 1:
+                        q += point if half > 0 else -point
+            part[k][bit] = q % R
+        for lv in (1, 2, 3, 4):
+            level(part[k], lv, 1 << (lv - 1))
+    last = [0] * parts
+    for k in range(blocks):
+        last[2 * k] = part[k][0]
+    for lv in (2, 3, 4):  # blocks k and k + 2^(lv - 2): 16 bits apart each
+        level(last, lv, 4 << lv)
+    return last[0]
 
 
 @pytest.mark.parametrize("trial", range(6))
