@@ -22,7 +22,8 @@
 //   merge heads  as in the plain pipeline
 //   reduction    per group of instances with the same c (one "window" each),
 //                the plain pipeline's reduction kernels on the group's buckets,
-//                then a gather into each instance's 254 results
+//                then one block per instance for the last levels and its 254
+//                results
 // The chain is captured once in a CUDA graph; every execution only writes the
 // instances' scalar and result pointers and replays the graph.
 #include "batch_tuning.h"

@@ -99,10 +99,11 @@ inline bool early_launches(cudaStream_t stream) {
   return status == cudaStreamCaptureStatusNone;
 }
 
-// Per-window sums of the reduction (reduce_groups_kernel, then one
-// reduce_level_kernel per level) for the p.windows windows of 2^(c-1) bucket
-// slots at `buckets`; afterwards streams[p.log_g & 1] holds each window's sums
-// for the gather kernels.  tree / streams: the ping-pong buffers of the plan.
+// The reduction (reduce_groups_kernel, then one reduce_level_kernel per level)
+// of the p.windows windows of 2^(c-1) bucket slots at `buckets`, up to level
+// tail_level(p.log_g): that many levels have run afterwards, and the window's
+// tree and streams are in tree[tail_level(p.log_g) & 1] and streams[the same],
+// for the tail kernel.  tree / streams: the ping-pong buffers of the plan.
 // behind_kernel: the stream's last operation is a kernel of the same call (see
 // launch_after).
 cudaError_t enqueue_window_sums(const plan &p, const xyzz *buckets, const uint8_t *flags, xyzz *const tree[2], xyzz *const streams[2],

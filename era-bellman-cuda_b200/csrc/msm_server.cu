@@ -60,8 +60,9 @@ struct slot {
   fork_set<cudaStream_t, cudaEvent_t> forks;
   bool busy = false;
   // Set by the completion host function, which must never wait for the
-  // server lock: the scheduler makes CUDA calls while holding it, and some of
-  // them wait for all device work, the host function included.
+  // server lock: a host function that waits holds up its stream and the
+  // runtime's other host functions, and whoever holds the lock may be waiting
+  // for those.
   std::atomic<bool> finished{false};
   std::vector<request *> members;
   size_t arena_offset = 0, arena_bytes = 0;

@@ -199,9 +199,11 @@ def test_batched_results(gpu, oracle):
 @pytest.mark.parametrize("bits", [[7], [8], [15, 16], [16], [31, 32], [32], [63, 64], [64], [127, 128], [128], [250, 253],
                                   [0, 1, 2, 4, 8, 16, 32, 64, 128], [15, 16, 31, 48, 80, 96, 112, 144, 176, 208, 240]])
 def test_doubling_chains(gpu, oracle, bits):
-    """Few finite results, at the edges of the tree's levels (four lanes per
-    doubling below 16 bits, a warp per point from there): chains of every
-    length, with and without an addition at their end; exact arithmetic."""
+    """Few finite results, at the edges of the tree's levels: chains of every
+    length, with and without an addition at their end; exact arithmetic.  In a
+    group of 16 bits the levels of 1 and 2 doublings (parts 1 and 2 apart) take
+    four lanes per point and those of 4 and 8 a warp per point; results from bit
+    128 on also go through the split and the levels across groups and blocks."""
     table = H.load_g_bases()
     rng = np.random.Generator(np.random.PCG64(sum(bits)))
     pts = {i: table[int(rng.integers(0, 256))] for i in bits}
